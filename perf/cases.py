@@ -8,7 +8,7 @@ A case is one of
            replays (up to 1024 tokens, as in the benchmark), else the plain call that a prefill makes.  `act` is the
            arithmetic: "w8a8" (FP8 tensor cores) or "w8a16" (the reference's: bf16 activations).
   experts  torch.ops.my_ops.fused_moe_fused_experts, the reference's op: routing done by the caller, per-slot rows out.
-           `weights` is "fp8" (with bf16 block scales, as checkpoints ship them) or "bf16" (scales = None).
+           `weights` is "fp8" (with fp32 block scales, as checkpoints ship them) or "bf16" (scales = None).
   mlp      torch.ops.my_ops.mlp_w8a8_quant_forward / mlp_w8a16_dq_forward: the dense FP8 MLP of a shared expert.
   linear   torch.ops.my_ops.mm_w8a16_dq_forward: one FP8 block-scaled projection.
 """
@@ -63,6 +63,13 @@ def _log_int(rng, lo, hi):
 
 
 def draw(rng):
+    while True:
+        c = _draw(rng)
+        if all({**c, "name": l["name"]} != l for l in listed()):  # another case than the listed ones
+            return c
+
+
+def _draw(rng):
     r = rng.random()
     if r < 0.55:
         shape = rng.choice(["small", "mixtral", "mixtral", "deepseek", "qwen"])
@@ -99,7 +106,7 @@ def _zipf_bias(E, seed):
     return 3.0 * np.log(p / p.sum())
 
 
-def _prepare_layer(c, seed):
+def _layer_parts(c, seed):
     s = SHAPES[c["shape"]]
     g = _gen(seed)
     T, E = c["tokens"], s["E"]
@@ -107,14 +114,19 @@ def _prepare_layer(c, seed):
     bias = torch.randn(E, generator=g, device=DEV) * 0.01 if s["score"] == "sigmoid" else None
     logit_bias = torch.from_numpy(_zipf_bias(E, seed)).float().to(DEV) if s.get("zipf") else None
     shared = W.random_experts(1, s["H"], s["shared"], DEV, seed=seed + 777) if s.get("shared") else None
-    cfg = MoEConfig(s["H"], s["I"], E, s["k"], s["score"], s.get("groups", 1), s.get("topk_groups", 1), True,
+    return _normal(g, T, s["H"]), wr, bias, logit_bias, W.random_experts(E, s["H"], s["I"], DEV, seed=seed), shared
+
+
+def _prepare_layer(c, seed):
+    s, T = SHAPES[c["shape"]], c["tokens"]
+    x, wr, bias, logit_bias, experts, shared = _layer_parts(c, seed)
+    cfg = MoEConfig(s["H"], s["I"], s["E"], s["k"], s["score"], s.get("groups", 1), s.get("topk_groups", 1), True,
                     s.get("scale", 1.0), s.get("shared", 0))
-    layer = FusedMoE(cfg, wr, *W.random_experts(E, s["H"], s["I"], DEV, seed=seed), bias=bias, shared=shared,
-                     logit_bias=logit_bias, max_tokens=T,
+    layer = FusedMoE(cfg, wr, *experts, bias=bias, shared=shared, logit_bias=logit_bias, max_tokens=T,
                      act_mode=L.ACT_W8A8 if c["act"] == "w8a8" else L.ACT_W8A16)
     if c["graph"]:
         layer.capture(T)
-    return {"call": layer.forward_graph if c["graph"] else layer.forward, "args": (_normal(g, T, s["H"]),)}
+    return {"call": layer.forward_graph if c["graph"] else layer.forward, "args": (x,)}
 
 
 def _prepare_experts(c, seed):
@@ -125,8 +137,8 @@ def _prepare_experts(c, seed):
         w = [(torch.randn(E, I, H, generator=g, device=DEV) * 0.02).to(torch.bfloat16) for _ in range(3)]
         scales = (None, None, None)
     else:
-        *w, sg, su, sd = W.random_experts(E, H, I, DEV, seed=seed)
-        scales = tuple(t.to(torch.bfloat16) for t in (sg, su, sd))
+        parts = W.random_experts(E, H, I, DEV, seed=seed)
+        w, scales = parts[:3], parts[3:]
     weight, ids = torch.randn(T, E, generator=g, device=DEV).softmax(-1).topk(k, dim=-1)
     weight = (weight / weight.sum(-1, keepdim=True)).to(torch.bfloat16)
     out = torch.empty(T, k, H, dtype=torch.bfloat16, device=DEV)
@@ -161,6 +173,84 @@ def run(state):
     return state["call"](*state["args"])
 
 
+# ---- the same arithmetic in 64 bits ---------------------------------------------------------------------------------
+# Roundings that belong to the arithmetic are kept (e4m3 activations with one scale per row and 128 columns; in w8a16
+# bf16 weights and bf16 intermediate results); every product, sum and activation between them is formed in 64 bits.
+def _q8(v):
+    """What a row means to the FP8 tensor cores: e4m3 values times a scale per 128 columns."""
+    g = v.unflatten(-1, (-1, 128))
+    amax = g.abs().amax(-1, keepdim=True).clamp_min(1e-12)
+    q = (g.float() * (448.0 / amax.float())).to(torch.float8_e4m3fn).double()
+    return (q * (amax.float() / 448.0).double()).flatten(-2)
+
+
+def _r16(v):
+    return v.to(torch.bfloat16).double()
+
+
+def _dequant(w, s):
+    return w.double() * s.double().repeat_interleave(128, 0)[:w.shape[0]].repeat_interleave(128, 1)
+
+
+def _exact_mlp(x, w, act):
+    """x [n,H] float64 -> [n,H]; w = gate, up, down [I,H] and their scales (None: bf16 weights)."""
+    if w[3] is None:
+        wg, wu, wd = (t.double() for t in w[:3])
+    else:
+        wg, wu, wd = (_dequant(t, sc) for t, sc in zip(w[:3], w[3:]))
+    if act == "w8a8":
+        x = _q8(x)
+        g, u = x @ wg.t(), x @ wu.t()
+        return _q8(g * torch.sigmoid(g) * u) @ wd
+    wg, wu, wd = _r16(wg), _r16(wu), _r16(wd)
+    g, u = _r16(x @ wg.t()), _r16(x @ wu.t())
+    return _r16(_r16(_r16(g * torch.sigmoid(g)) * u) @ wd)
+
+
+def _exact_slots(x, ids, experts, act):
+    T, k = ids.shape
+    out = torch.zeros(T, k, x.shape[1], dtype=torch.float64, device=DEV)
+    for e in torch.unique(ids).tolist():
+        t, j = (ids == e).nonzero(as_tuple=True)
+        out[t, j] = _exact_mlp(x[t], [w if w is None else w[e] for w in experts], act)
+    return out
+
+
+def _exact_layer(c, seed):
+    s = SHAPES[c["shape"]]
+    x, wr, bias, logit_bias, experts, shared = _layer_parts(c, seed)
+    x = x.double()
+    logits = x @ wr.double().t()
+    if logit_bias is not None:
+        logits = logits + logit_bias.double()
+    score = logits.softmax(-1) if s["score"] == "softmax" else logits.sigmoid()
+    sel = score if bias is None else score + bias.double()
+    if s.get("groups", 1) > 1:
+        g = sel.unflatten(-1, (s["groups"], -1))
+        keep = g.topk(2, -1).values.sum(-1).topk(s["topk_groups"], -1).indices
+        mask = torch.zeros_like(g[..., 0]).scatter_(-1, keep, 1.0).bool()
+        sel = g.masked_fill(~mask.unsqueeze(-1), -math.inf).flatten(-2)
+    ids = sel.topk(s["k"], -1).indices
+    w = score.gather(-1, ids)
+    w = w / w.sum(-1, keepdim=True) * s.get("scale", 1.0)
+    out = (w.unsqueeze(-1) * _exact_slots(x, ids, experts, c["act"])).sum(1)
+    return out if shared is None else out + _exact_mlp(x, [t[0] for t in shared], c["act"])
+
+
+def exact(case, seed):
+    c = case
+    seed = int(seed) % (1 << 31)
+    if c["path"] == "layer":
+        return _exact_layer(c, seed)
+    args = prepare(c, seed)["args"]
+    if c["path"] == "experts":  # args: out, x, -, -, three weights, three scales, ids, ...
+        return _exact_slots(args[1].double(), args[10], args[4:10], "w8a16" if c["weights"] == "bf16" else "w8a8")
+    if c["path"] == "mlp":
+        return _exact_mlp(args[0].double(), args[1:7], c["act"])
+    x, w, scale = args[:3]
+    return _q8(x.double()) @ _dequant(w, scale).t()
+
+
 # ---- what a pass cannot do without ---------------------------------------------------------------------------------
 def _activated(s, T):
     """Experts that T tokens activate.  Even routing: its expectation.  Skewed routing: counted on a sample of logits
@@ -187,7 +277,7 @@ def work(case):
     flops = 6.0 * T * k * H * I + 6.0 * T * H * Is
     if case["path"] == "experts":  # routing given, even; per-slot rows out
         act = E * (1.0 - (1.0 - k / E) ** T)
-        per = 6 * H * I if case["weights"] == "bf16" else 3 * H * I + 6 * (H // 128) * (I // 128)
+        per = 6 * H * I if case["weights"] == "bf16" else 3 * H * I + 12 * (H // 128) * (I // 128)
         return {"bytes": act * per + 2 * T * H + 2 * T * k * H + 6 * T * k, "flops": flops}
     per = 3 * H * I + 12 * (H // 128) * (I // 128)
     shared = 3 * H * Is + 12 * (H // 128) * (Is // 128)
