@@ -33,6 +33,23 @@ def test_op_noaux_tc_topk_like_reference_test(m):
         torch.ops.my_ops.noaux_tc_topk(values.cpu(), indices.cpu(), scores, 8, 4, 8)
 
 
+def test_op_bf16_scales_are_read_on_every_call(m):
+    """New scale values in memory that held others before (a freed and reused block, a write through .data) count."""
+    T, H, I, E, k = 16, 256, 256, 4, 2
+    p = small_problem(T, H, I, E, k, seed=17, scale_dtype=torch.bfloat16)
+    p["rw"] = p["w"].to(torch.bfloat16)
+    d = to_dev(p)
+    out = torch.empty(T, k, H, dtype=torch.bfloat16, device=DEV)
+    for f in (1.0, 2.0):
+        for n in ("sg", "su", "sd"):
+            p[n] = (p[n].float() * f).to(torch.bfloat16)
+            d[n].data.copy_(p[n])  # same address, size and version counter
+        _call_v1(out, d, E, k)
+        want = O.experts_w8a8(p["x"], p["ids"], p["wg"], p["wu"], p["wd"], p["sg"], p["su"], p["sd"])
+        met = O.parity_metrics(out, want)
+        assert met["max_rel"] <= 2e-2 and met["cosine"] >= 0.9995, (f, met)
+
+
 def _call_v1(out, d, E, k):
     return torch.ops.my_ops.fused_moe_fused_experts(
         out, d["x"], None, None, d["wg"], d["wu"], d["wd"], d["sg"], d["su"], d["sd"], d["ids"], d["rw"],

@@ -187,26 +187,6 @@ bool check_status_from_env() {
   return v && v[0] == '1';
 }
 
-// fp32 copies of bf16 block scales, made once per scale tensor (keyed by storage address, size and version counter)
-// instead of on every call: the tensor-core kernels read fp32 scales only.
-Tensor scales_as_f32(const Tensor& s) {
-  if (s.scalar_type() == kFloat) return s;
-  struct Entry {
-    int64_t numel;
-    uint32_t version;
-    Tensor f32;
-  };
-  static std::mutex mu;
-  static std::unordered_map<const void*, Entry> cache;
-  std::lock_guard<std::mutex> lock(mu);
-  auto it = cache.find(s.data_ptr());
-  if (it == cache.end() || it->second.numel != s.numel() || it->second.version != s._version()) {
-    if (cache.size() > 64) cache.clear();
-    it = cache.insert_or_assign(s.data_ptr(), Entry{s.numel(), (uint32_t)s._version(), s.to(kFloat)}).first;
-  }
-  return it->second.f32;
-}
-
 // bf16-weight experts (scales = None in the reference call, python/test/fused_moe_bf16.py:113-122): same pipeline,
 // the bf16 tensor-core kernels read the weights as they are
 Tensor run_experts_bf16(Tensor& output, const Tensor& input, const Tensor& gate_w, const Tensor& up_w,
@@ -295,10 +275,6 @@ Tensor run_experts(Tensor& output, const Tensor& input, const Tensor& gate_w, co
               "select_experts must be [T,k]");
   TORCH_CHECK(routing_weights.numel() == T * top_k, "routing_weights must be [T,k]");
 
-  // the FP8 tensor-core path reads fp32 scales: convert bf16 ones once per tensor, not per call
-  const bool to_f32 = act_mode == B200MOE_ACT_W8A8 && gate_s.scalar_type() == kBFloat16;
-  const Tensor gs = to_f32 ? scales_as_f32(gate_s) : gate_s, us = to_f32 ? scales_as_f32(up_s) : up_s,
-               ds = to_f32 ? scales_as_f32(down_s) : down_s;
   b200moe_experts_desc d{};
   d.T = T;
   d.H = H;
@@ -315,7 +291,7 @@ Tensor run_experts(Tensor& output, const Tensor& input, const Tensor& gate_w, co
   }
   d.act_mode = act_mode;
   d.impl = B200MOE_IMPL_AUTO;
-  d.scale_dtype = scale_dtype_of(gs);
+  d.scale_dtype = scale_dtype_of(gate_s);
   if (routing_weights.scalar_type() == kFloat) d.w_dtype = B200MOE_F32;
   else if (routing_weights.scalar_type() == kBFloat16) d.w_dtype = B200MOE_BF16;
   else TORCH_CHECK(false, "routing_weights must be float32 or bfloat16");
@@ -329,7 +305,7 @@ Tensor run_experts(Tensor& output, const Tensor& input, const Tensor& gate_w, co
   const size_t ws_bytes = (size_t)ws.numel() - (reinterpret_cast<char*>(wsp) - reinterpret_cast<char*>(ws.data_ptr()));
   Tensor status = status_word(input.device());
   int rc = b200moe_experts(output.data_ptr(), input.data_ptr(), gate_w.data_ptr(), up_w.data_ptr(),
-                           down_w.data_ptr(), gs.data_ptr(), us.data_ptr(), ds.data_ptr(),
+                           down_w.data_ptr(), gate_s.data_ptr(), up_s.data_ptr(), down_s.data_ptr(),
                            select_experts.data_ptr<int32_t>(), routing_weights.data_ptr(), nullptr, nullptr,
                            nullptr, nullptr, nullptr, nullptr, &d, wsp, ws_bytes, status.data_ptr<int32_t>(), st);
   check_rc(rc, "b200moe_experts");
