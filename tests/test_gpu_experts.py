@@ -240,3 +240,28 @@ def test_capped_grid_gives_the_same_result(m):
     assert torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2])
     with pytest.raises(Exception):
         m.ops.experts(outs[0], d["x"], d["wg"], d["wu"], d["wd"], d["sg"], d["su"], d["sd"], d["ids"], max_ctas=-1)
+
+
+@pytest.mark.parametrize("factor", [2.0 ** -20, 1.0, 2.0 ** 12, 2.0 ** 22])
+def test_w8a16_dequantisation_over_the_scale_range(m, factor):
+    """The tensor-core dequantisation against
+    the CUDA-core kernels, which convert value by value: both round w * scale to bf16 once, so the down projection of
+    one-hot rows agrees to the bf16 rounding of h and of the sum (2^-8), and a NaN weight reaches the same columns."""
+    L = m.lib
+    T, H, I, E, k = 40, 384, 256, 4, 2
+    p = small_problem(T, H, I, E, k, seed=31)
+    p["sd"] = p["sd"] * factor
+    p["wd"].view(torch.uint8)[1, 3, 200] = 0x7F   # NaN
+    p["wd"].view(torch.uint8)[2, 5, 7] = 0xFF     # -NaN
+    p["wd"].view(torch.uint8)[0, :, 5] = 0x01     # smallest subnormal
+    d = to_dev(p)
+    outs = []
+    for impl in (L.IMPL_SIMPLE, L.IMPL_TCGEN05):
+        out = torch.zeros(T, k, H, dtype=torch.bfloat16, device=DEV)
+        m.ops.experts(out, d["x"], d["wg"], d["wu"], d["wd"], d["sg"], d["su"], d["sd"], d["ids"],
+                      act_mode=L.ACT_W8A16, impl=impl)
+        outs.append(out.float().cpu())
+    nan = torch.isnan(outs[0])
+    assert nan.any() and torch.equal(nan, torch.isnan(outs[1]))
+    a, b = outs[0][~nan], outs[1][~nan]
+    assert (a - b).norm() <= 2.0 ** -8 * a.norm()
