@@ -33,7 +33,7 @@ int choose_ksplit(int64_t P, int64_t E, int64_t H, int64_t I) {
 }
 
 struct WsLayout {
-  size_t offsets, sorted, scratch, mtiles, nmt, xq, xs, hq, hs, y, sc32, s_sc32, y32, s_y32, acc32;
+  size_t offsets, sorted, pos_of, scratch, mtiles, nmt, xq, xs, hq, hs, y, sc32, s_sc32, y32, s_y32, acc32;
   size_t s_offsets, s_mtiles, s_nmt, s_xq, s_xs, s_hq, s_hs, s_y;
   size_t total;
   int64_t P, ld, lds;
@@ -58,6 +58,7 @@ WsLayout make_layout(const b200moe_experts_desc& d) {
   const size_t nH = d.H / kBlock, nI = d.I / kBlock;
   L.offsets = take((d.E + 1) * sizeof(int32_t));
   L.sorted = take((size_t)P * sizeof(int32_t));
+  L.pos_of = take((size_t)P * sizeof(int32_t));
   L.scratch = take(b200moe_permute_scratch_ints(P, d.E) * sizeof(int32_t));
   L.mtiles = take((size_t)L.max_mtiles * 2 * sizeof(int32_t));
   L.nmt = take(sizeof(int32_t));
@@ -224,8 +225,8 @@ extern "C" int b200moe_experts(void* out, const void* x, const void* w_gate, con
 
   if (do_prep) {
     bool tiles_done = false;
-    rc = moe_permute_impl(I32(L.sorted), I32(L.offsets), ids, d->T, d->k, d->E, I32(L.scratch), status, I32(L.mtiles),
-                          I32(L.nmt), L.max_mtiles, &tiles_done, stream);
+    rc = moe_permute_impl(I32(L.sorted), I32(L.offsets), ids, d->T, d->k, d->E, I32(L.scratch), status, I32(L.pos_of),
+                          I32(L.mtiles), I32(L.nmt), L.max_mtiles, &tiles_done, stream);
     if (rc) return rc;
     if (!tiles_done) {
       rc = moe_build_mtiles(I32(L.mtiles), I32(L.nmt), I32(L.offsets), (int)d->E, L.P, L.max_mtiles, st);
@@ -233,8 +234,8 @@ extern "C" int b200moe_experts(void* out, const void* x, const void* w_gate, con
     }
   }
   if (w8a8 && do_prep) {
-    rc = b200moe_quant_rows(reinterpret_cast<uint8_t*>(ws + L.xq), reinterpret_cast<float*>(ws + L.xs), L.ld,
-                            x, I32(L.sorted), d->k, L.P, d->H, stream);
+    rc = moe_quant_tokens(reinterpret_cast<uint8_t*>(ws + L.xq), reinterpret_cast<float*>(ws + L.xs), L.ld, x,
+                          I32(L.pos_of), d->T, d->k, d->H, st);
     if (rc) return rc;
   }
 
@@ -331,14 +332,10 @@ extern "C" int b200moe_experts(void* out, const void* x, const void* w_gate, con
   if (d->I_shared > 0) {
     cudaStream_t ss = side ? side->s : st;
     if (do_prep) {
-      rc = moe_fill_identity_offsets(I32(L.s_offsets), d->T, ss);
-      if (rc) return rc;
-      rc = moe_build_mtiles(I32(L.s_mtiles), I32(L.s_nmt), I32(L.s_offsets), 1, d->T, L.s_max_mtiles, ss);
-      if (rc) return rc;
-    }
-    if (w8a8 && do_prep) {
-      rc = b200moe_quant_rows(reinterpret_cast<uint8_t*>(ws + L.s_xq), reinterpret_cast<float*>(ws + L.s_xs),
-                              L.lds, x, nullptr, 1, d->T, d->H, (void*)ss);
+      const MoeIdentityLists lists{I32(L.s_offsets), I32(L.s_mtiles), I32(L.s_nmt)};
+      rc = w8a8 ? moe_quant_identity(reinterpret_cast<uint8_t*>(ws + L.s_xq), reinterpret_cast<float*>(ws + L.s_xs),
+                                     L.lds, x, d->T, d->H, lists, ss)
+                : moe_identity_lists(lists, d->T, ss);
       if (rc) return rc;
     }
     const int64_t nscs = (d->I_shared / kBlock) * (d->H / kBlock);
@@ -619,12 +616,8 @@ extern "C" int b200moe_linear_w8(void* out, const void* x, const void* w, const 
   int32_t* offsets = reinterpret_cast<int32_t*>(ws + L.offsets);
   int32_t* mtiles = reinterpret_cast<int32_t*>(ws + L.mtiles);
   int32_t* nmt = reinterpret_cast<int32_t*>(ws + L.nmt);
-  int rc = moe_fill_identity_offsets(offsets, M, st);
-  if (rc) return rc;
-  rc = moe_build_mtiles(mtiles, nmt, offsets, 1, M, L.max_mtiles, st);
-  if (rc) return rc;
-  rc = b200moe_quant_rows(reinterpret_cast<uint8_t*>(ws + L.xq), reinterpret_cast<float*>(ws + L.xs), L.ld, x, nullptr,
-                          1, M, K, stream);
+  int rc = moe_quant_identity(reinterpret_cast<uint8_t*>(ws + L.xq), reinterpret_cast<float*>(ws + L.xs), L.ld, x, M, K,
+                              MoeIdentityLists{offsets, mtiles, nmt}, st);
   if (rc) return rc;
   const void* sc = scale;
   if (scale_dtype == B200MOE_BF16) {
@@ -711,9 +704,7 @@ extern "C" int b200moe_scaled_mm(void* out, int out_dtype, const void* a, const 
   int32_t* offsets = reinterpret_cast<int32_t*>(ws + L.offsets);
   int32_t* mtiles = reinterpret_cast<int32_t*>(ws + L.mtiles);
   int32_t* nmt = reinterpret_cast<int32_t*>(ws + L.nmt);
-  int rc = moe_fill_identity_offsets(offsets, M, st);
-  if (rc) return rc;
-  rc = moe_build_mtiles(mtiles, nmt, offsets, 1, M, L.max_mtiles, st);
+  int rc = moe_identity_lists(MoeIdentityLists{offsets, mtiles, nmt}, M, st);
   if (rc) return rc;
   // the kernel applies act_scale[row,kb] * weight_scale[nb,kb] to every 128-deep partial sum: constant grids here
   const int64_t nxs = (K / kBlock) * L.ld, nws = ((N + kBlock - 1) / kBlock) * (K / kBlock);

@@ -47,15 +47,37 @@ struct MoeGemmArgs {
   int32_t* status;
 };
 
-// b200moe_permute that also writes the m-tile list when one CTA does the whole sort (at most 1024 pairs)
+// lists of an identity problem (one expert, rows 0..rows): offsets = {0, rows} and its m-tiles; offsets NULL = none
+struct MoeIdentityLists {
+  int32_t* offsets;
+  int32_t* mtiles;
+  int32_t* num_mtiles;
+};
+#ifdef __CUDACC__
+// by the threads of one block
+__device__ __forceinline__ void moe_write_identity_lists(const MoeIdentityLists& l, int rows) {
+  const int n = (rows + kTileM - 1) / kTileM;
+  for (int i = threadIdx.x; i < n; i += blockDim.x) {
+    l.mtiles[2 * i] = 0;
+    l.mtiles[2 * i + 1] = i * kTileM;
+  }
+  if (threadIdx.x == 0) l.offsets[0] = 0, l.offsets[1] = rows, *l.num_mtiles = n;
+}
+#endif
+
+// b200moe_permute that also writes the inverse map (pos_of, may be NULL) and the m-tile list when one CTA does the whole sort (at most 1024 pairs)
 int moe_permute_impl(int32_t* sorted_pair, int32_t* expert_offsets, const int32_t* ids, int64_t T, int64_t k, int64_t E,
-                     int32_t* scratch, int32_t* status, int32_t* mtiles, int32_t* num_mtiles, int max_mtiles,
-                     bool* tiles_done, void* stream);
+                     int32_t* scratch, int32_t* status, int32_t* pos_of, int32_t* mtiles, int32_t* num_mtiles,
+                     int max_mtiles, bool* tiles_done, void* stream);
+// quantised rows of x at the positions of every token's k pairs; quantised rows 0..rows with the identity lists
+int moe_quant_tokens(uint8_t* q, float* s_t, int64_t ld, const void* x, const int32_t* pos_of, int64_t T, int64_t k,
+                     int64_t H, cudaStream_t st);
+int moe_quant_identity(uint8_t* q, float* s_t, int64_t ld, const void* x, int64_t rows, int64_t H,
+                       const MoeIdentityLists& lists, cudaStream_t st);
 // tiles of rows [offsets[e], offsets[e+1]) clipped to max_rows; at most max_mtiles entries are written
 int moe_build_mtiles(int32_t* mtiles, int32_t* num_mtiles, const int32_t* offsets, int E, int64_t max_rows,
                      int max_mtiles, cudaStream_t st);
-// identity problem (one expert, rows 0..T): offsets = {0,T}
-int moe_fill_identity_offsets(int32_t* offsets, int64_t T, cudaStream_t st);
+int moe_identity_lists(const MoeIdentityLists& lists, int64_t rows, cudaStream_t st);
 
 int moe_gemm1_simple(const MoeGemmArgs& a, int act_mode, cudaStream_t st);
 int moe_gemm2_simple(const MoeGemmArgs& a, int act_mode, cudaStream_t st);

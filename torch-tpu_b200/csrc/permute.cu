@@ -8,13 +8,12 @@
 //   scatter : position = offsets[e] + chunk_base[c][e] + (pairs of e in earlier warps of the chunk)
 //             + (pairs of e in lower lanes of the warp)
 // For P <= 1024 all three steps run in one single-CTA kernel.
-#include "common.cuh"
+#include "internal.h"
 
 namespace {
 
 constexpr int kChunk = 1024;  // pairs per CTA (32 warps)
 constexpr int kMaxE = 1024;
-constexpr int kRowsPerTile = 128;  // rows of one m-tile of the grouped GEMMs
 constexpr int kMaxDevices = 64;  // per-device caches below are indexed by the CUDA device ordinal
 
 // Per-warp histogram of this chunk in shared memory: wh[w*E + e].  Returns the pair's expert (or -1)
@@ -92,7 +91,7 @@ permute_scan_kernel(int32_t* __restrict__ chunk_cnt, int nchunks, int E, int32_t
 __global__ void __launch_bounds__(kChunk)
 permute_scatter_kernel(const int32_t* __restrict__ ids, int64_t P, int E,
                        const int32_t* __restrict__ chunk_base, const int32_t* __restrict__ offsets,
-                       int32_t* __restrict__ sorted_pair) {
+                       int32_t* __restrict__ sorted_pair, int32_t* __restrict__ pos_of) {
   extern __shared__ int wh[];
   int rank;
   const int64_t p = (int64_t)blockIdx.x * kChunk + threadIdx.x;
@@ -107,10 +106,12 @@ permute_scatter_kernel(const int32_t* __restrict__ ids, int64_t P, int E,
     }
   }
   __syncthreads();
+  int pos = -1;
   if (e >= 0) {
-    int pos = offsets[e] + chunk_base[(int64_t)blockIdx.x * E + e] + wh[(threadIdx.x >> 5) * E + e] + rank;
+    pos = offsets[e] + chunk_base[(int64_t)blockIdx.x * E + e] + wh[(threadIdx.x >> 5) * E + e] + rank;
     sorted_pair[pos] = (int32_t)p;
   }
+  if (pos_of && p < P) pos_of[p] = pos;
   // Pairs whose id was out of range have no position: the tail [offsets[E], P) is filled with -1 so that no consumer
   // ever indexes with an unwritten entry (valid positions all lie below offsets[E], so this does not race with them).
   if (p < P && p >= offsets[E]) sorted_pair[p] = -1;
@@ -120,7 +121,7 @@ permute_scatter_kernel(const int32_t* __restrict__ ids, int64_t P, int E,
 __global__ void __launch_bounds__(kChunk)
 permute_small_kernel(const int32_t* __restrict__ ids, int64_t P, int E, int32_t* __restrict__ offsets,
                      int32_t* __restrict__ sorted_pair, int32_t* status, int32_t* __restrict__ mtiles,
-                     int32_t* __restrict__ num_mtiles, int max_mtiles) {
+                     int32_t* __restrict__ num_mtiles, int max_mtiles, int32_t* __restrict__ pos_of) {
   extern __shared__ int wh[];
   __shared__ int tmp[kChunk];
   __shared__ int soffs[kMaxE + 1];
@@ -138,7 +139,12 @@ permute_small_kernel(const int32_t* __restrict__ ids, int64_t P, int E, int32_t*
   block_exclusive_scan(total, E, soffs, tmp);
   __syncthreads();
   for (int i = threadIdx.x; i <= E; i += blockDim.x) offsets[i] = soffs[i];
-  if (e >= 0) sorted_pair[soffs[e] + wh[(threadIdx.x >> 5) * E + e] + rank] = (int32_t)threadIdx.x;
+  int pos = -1;
+  if (e >= 0) {
+    pos = soffs[e] + wh[(threadIdx.x >> 5) * E + e] + rank;
+    sorted_pair[pos] = (int32_t)threadIdx.x;
+  }
+  if (pos_of && (int64_t)threadIdx.x < P) pos_of[threadIdx.x] = pos;
   if ((int64_t)threadIdx.x < P && (int)threadIdx.x >= soffs[E]) sorted_pair[threadIdx.x] = -1;  // dropped pairs: see above
   if (mtiles) {
     // the m-tile list of the grouped GEMMs ({expert, first row} per 128 rows of an expert) from the same offsets:
@@ -146,13 +152,13 @@ permute_small_kernel(const int32_t* __restrict__ ids, int64_t P, int E, int32_t*
     __syncthreads();
     const int t = threadIdx.x;
     const int b = t < E ? soffs[t] : 0;
-    const int n = t < E ? (soffs[t + 1] - b + kRowsPerTile - 1) / kRowsPerTile : 0;
+    const int n = t < E ? (soffs[t + 1] - b + kTileM - 1) / kTileM : 0;
     __shared__ int toffs[kMaxE + 1];
     block_exclusive_scan(n, E, toffs, tmp);
     __syncthreads();
     for (int i = 0; i < n && toffs[t] + i < max_mtiles; ++i) {
       mtiles[2 * (toffs[t] + i)] = t;
-      mtiles[2 * (toffs[t] + i) + 1] = b + i * kRowsPerTile;
+      mtiles[2 * (toffs[t] + i) + 1] = b + i * kTileM;
     }
     if (t == 0) *num_mtiles = min(toffs[E], max_mtiles);
   }
@@ -181,7 +187,8 @@ __global__ void gather_scatter_index_kernel(int32_t* __restrict__ gather_index,
 __global__ void __launch_bounds__(256)
 quant_rows_kernel(uint8_t* __restrict__ q, float* __restrict__ s_t, int64_t ld,
                   const __nv_bfloat16* __restrict__ x, const int32_t* __restrict__ row_map, int div,
-                  int64_t rows, int H, int cpw, int warps_per_row) {
+                  int64_t rows, int H, int cpw, int warps_per_row, MoeIdentityLists lists) {
+  if (lists.offsets && blockIdx.x == 0) moe_write_identity_lists(lists, (int)rows);
   const int lane = threadIdx.x & 31;
   const int64_t w = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
   const int64_t r = w / warps_per_row;
@@ -229,6 +236,71 @@ quant_rows_kernel(uint8_t* __restrict__ q, float* __restrict__ s_t, int64_t ld,
   }
 }
 
+// The routed rows of a layer, token by token: a token is read and quantised ONCE and its e4m3 bytes are stored to the
+// positions of its k (token,slot) pairs (pos_of, the inverse of the permutation; -1 = dropped).  Walking the sorted rows
+// instead reads and converts every token k times: Qwen3 shape, 8192 tokens x 8 slots: 72 us, bound by the conversions
+// and k-fold reads, for 134 MB of output that the copy bandwidth writes in 20 us; Mixtral 4096 tokens 21 us.
+// A lane owns 16 consecutive columns (eight lanes one 128-column group), so a store instruction puts down 512 bytes of a
+// row; a warp takes `cpw` 512-column chunks of a token, their loads issued together.
+constexpr int QT_CPW = 2;
+__global__ void __launch_bounds__(256)
+quant_tokens_kernel(uint8_t* __restrict__ q, float* __restrict__ s_t, int64_t ld, const __nv_bfloat16* __restrict__ x,
+                    const int32_t* __restrict__ pos_of, int64_t T, int k, int H, int cpw, int warps_per_tok) {
+  const int lane = threadIdx.x & 31;
+  const int64_t w = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
+  const int64_t t = w / warps_per_tok;
+  if (t >= T) return;  // uniform over the warp
+  const int c0 = (int)(w - t * warps_per_tok) * cpw * 512 + lane * 16;
+  uint4 raw[QT_CPW][2];
+#pragma unroll
+  for (int u = 0; u < QT_CPW; ++u) {
+    const int c = c0 + u * 512;
+    const bool on = u < cpw && c < H;
+    raw[u][0] = on ? *reinterpret_cast<const uint4*>(x + t * H + c) : make_uint4(0, 0, 0, 0);
+    raw[u][1] = on ? *reinterpret_cast<const uint4*>(x + t * H + c + 8) : make_uint4(0, 0, 0, 0);
+  }
+  int32_t my_pos = lane < k ? pos_of[t * k + lane] : -1;
+  uint4 out[QT_CPW];
+  float sc[QT_CPW];
+#pragma unroll
+  for (int u = 0; u < QT_CPW; ++u) {
+    float v[16], amax = 0.f;
+    const __nv_bfloat162* b2 = reinterpret_cast<const __nv_bfloat162*>(&raw[u][0]);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const float2 f = __bfloat1622float2(b2[i]);
+      v[2 * i] = f.x;
+      v[2 * i + 1] = f.y;
+      amax = fmaxf(amax, fmaxf(fabsf(f.x), fabsf(f.y)));
+    }
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+    amax = fmaxf(amax, kAmaxFloor);
+    const float inv = kFp8Max / amax;
+    sc[u] = amax / kFp8Max;
+    out[u].x = moe_f32x4_to_e4m3x4(v[0] * inv, v[1] * inv, v[2] * inv, v[3] * inv);
+    out[u].y = moe_f32x4_to_e4m3x4(v[4] * inv, v[5] * inv, v[6] * inv, v[7] * inv);
+    out[u].z = moe_f32x4_to_e4m3x4(v[8] * inv, v[9] * inv, v[10] * inv, v[11] * inv);
+    out[u].w = moe_f32x4_to_e4m3x4(v[12] * inv, v[13] * inv, v[14] * inv, v[15] * inv);
+  }
+  for (int j0 = 0; j0 < k; j0 += 32) {
+    if (j0 > 0) my_pos = j0 + lane < k ? pos_of[t * k + j0 + lane] : -1;
+    const int n = min(32, k - j0);
+    for (int j = 0; j < n; ++j) {
+      const int64_t p = __shfl_sync(0xffffffffu, my_pos, j);
+      if (p < 0) continue;
+#pragma unroll
+      for (int u = 0; u < QT_CPW; ++u) {
+        const int c = c0 + u * 512;
+        if (u < cpw && c < H) {
+          *reinterpret_cast<uint4*>(q + p * H + c) = out[u];
+          if ((lane & 7) == 0) s_t[(int64_t)(c >> 7) * ld + p] = sc[u];
+        }
+      }
+    }
+  }
+}
+
 }  // namespace
 
 extern "C" size_t b200moe_permute_scratch_ints(int64_t P, int64_t E) {
@@ -236,11 +308,11 @@ extern "C" size_t b200moe_permute_scratch_ints(int64_t P, int64_t E) {
   return (size_t)((P + kChunk - 1) / kChunk) * (size_t)E;
 }
 
-// b200moe_permute; with `mtiles` != NULL and at most 1024 pairs the one-CTA kernel writes the GEMMs' m-tile list too and
+// b200moe_permute; with `pos_of` != NULL the inverse map too (pos_of[pair] = its position, -1 = dropped); with `mtiles` != NULL and at most 1024 pairs the one-CTA kernel writes the GEMMs' m-tile list too and
 // *tiles_done is set (else the caller builds the list from expert_offsets)
 int moe_permute_impl(int32_t* sorted_pair, int32_t* expert_offsets, const int32_t* ids, int64_t T, int64_t k, int64_t E,
-                     int32_t* scratch, int32_t* status, int32_t* mtiles, int32_t* num_mtiles, int max_mtiles,
-                     bool* tiles_done, void* stream) {
+                     int32_t* scratch, int32_t* status, int32_t* pos_of, int32_t* mtiles, int32_t* num_mtiles,
+                     int max_mtiles, bool* tiles_done, void* stream) {
   if (tiles_done) *tiles_done = false;
   MOE_CHECK_ARG(sorted_pair && expert_offsets && ids && T >= 0 && k > 0 && E > 0);
   const int64_t P = T * k;
@@ -259,7 +331,7 @@ int moe_permute_impl(int32_t* sorted_pair, int32_t* expert_offsets, const int32_
   }
   if (P <= kChunk) {
     permute_small_kernel<<<1, kChunk, smem, st>>>(ids, P, (int)E, expert_offsets, sorted_pair, status, mtiles,
-                                                  num_mtiles, max_mtiles);
+                                                  num_mtiles, max_mtiles, pos_of);
     if (tiles_done) *tiles_done = mtiles != nullptr;
     return moe_launch_status();
   }
@@ -267,14 +339,15 @@ int moe_permute_impl(int32_t* sorted_pair, int32_t* expert_offsets, const int32_
   const int nchunks = (int)((P + kChunk - 1) / kChunk);
   permute_hist_kernel<<<nchunks, kChunk, smem, st>>>(ids, P, (int)E, scratch, status);
   permute_scan_kernel<<<1, kChunk, 0, st>>>(scratch, nchunks, (int)E, expert_offsets);
-  permute_scatter_kernel<<<nchunks, kChunk, smem, st>>>(ids, P, (int)E, scratch, expert_offsets, sorted_pair);
+  permute_scatter_kernel<<<nchunks, kChunk, smem, st>>>(ids, P, (int)E, scratch, expert_offsets, sorted_pair,
+                                                        pos_of);
   return moe_launch_status();
 }
 
 extern "C" int b200moe_permute(int32_t* sorted_pair, int32_t* expert_offsets, const int32_t* ids, int64_t T,
                                int64_t k, int64_t E, int32_t* scratch, int32_t* status, void* stream) {
-  return moe_permute_impl(sorted_pair, expert_offsets, ids, T, k, E, scratch, status, nullptr, nullptr, 0, nullptr,
-                          stream);
+  return moe_permute_impl(sorted_pair, expert_offsets, ids, T, k, E, scratch, status, nullptr, nullptr, nullptr, 0,
+                          nullptr, stream);
 }
 
 extern "C" int b200moe_gather_scatter_index(int32_t* gather_index, int32_t* scatter_index,
@@ -289,17 +362,40 @@ extern "C" int b200moe_gather_scatter_index(int32_t* gather_index, int32_t* scat
   return moe_launch_status();
 }
 
+namespace {
+int launch_quant_rows(uint8_t* q, float* s_t, int64_t ld, const void* x, const int32_t* row_map, int64_t div, int64_t rows,
+                      int64_t H, const MoeIdentityLists& lists, cudaStream_t st) {
+  const int chunks = (int)((H + 255) / 256);
+  const int cpw = rows >= 2048 ? chunks : 1;
+  const int warps_per_row = (chunks + cpw - 1) / cpw;
+  quant_rows_kernel<<<(unsigned)((rows * warps_per_row + 7) / 8), 256, 0, st>>>(
+      q, s_t, ld, reinterpret_cast<const __nv_bfloat16*>(x), row_map, (int)div, rows, (int)H, cpw, warps_per_row, lists);
+  return moe_launch_status();
+}
+}  // namespace
+
 extern "C" int b200moe_quant_rows(uint8_t* q, float* s_t, int64_t ld, const void* x, const int32_t* row_map,
                                   int64_t div, int64_t rows, int64_t H, void* stream) {
   MOE_CHECK_ARG(q && s_t && x && rows >= 0 && H > 0 && div > 0 && ld >= rows);
   MOE_CHECK_SHAPE(H % kBlock == 0);
   if (!moe_aligned16(x) || !moe_aligned16(q)) return B200MOE_EALIGN;
   if (rows == 0) return B200MOE_OK;
-  const int chunks = (int)((H + 255) / 256);
-  const int cpw = rows >= 2048 ? chunks : 1;
-  const int warps_per_row = (chunks + cpw - 1) / cpw;
-  quant_rows_kernel<<<(unsigned)((rows * warps_per_row + 7) / 8), 256, 0, (cudaStream_t)stream>>>(
-      q, s_t, ld, reinterpret_cast<const __nv_bfloat16*>(x), row_map, (int)div, rows, (int)H, cpw, warps_per_row);
+  return launch_quant_rows(q, s_t, ld, x, row_map, div, rows, H, MoeIdentityLists{}, (cudaStream_t)stream);
+}
+
+int moe_quant_identity(uint8_t* q, float* s_t, int64_t ld, const void* x, int64_t rows, int64_t H,
+                       const MoeIdentityLists& lists, cudaStream_t st) {
+  return launch_quant_rows(q, s_t, ld, x, nullptr, 1, rows, H, lists, st);
+}
+
+int moe_quant_tokens(uint8_t* q, float* s_t, int64_t ld, const void* x, const int32_t* pos_of, int64_t T, int64_t k,
+                     int64_t H, cudaStream_t st) {
+  const int64_t chunks = (H + 511) / 512;
+  // two chunks per warp once that still leaves every SM its full set of warps
+  const int cpw = T * chunks >= 2 * 64 * 148 ? QT_CPW : 1;
+  const int64_t wpt = (chunks + cpw - 1) / cpw;
+  quant_tokens_kernel<<<(unsigned)((T * wpt + 7) / 8), 256, 0, st>>>(
+      q, s_t, ld, reinterpret_cast<const __nv_bfloat16*>(x), pos_of, T, (int)k, (int)H, cpw, (int)wpt);
   return moe_launch_status();
 }
 
