@@ -8,7 +8,7 @@
 #include <limits.h>
 #include <math.h>
 
-#include "common.cuh"
+#include "internal.h"
 
 namespace {
 
@@ -26,32 +26,41 @@ __device__ __forceinline__ void warp_argmax(float& v, int& idx) {
   }
 }
 
+// A float as an unsigned number of the same order (-0 counts as +0, NaN above everything), so that a warp's maximum is
+// one redux instruction.
+__device__ __forceinline__ uint32_t order_key(float v) {
+  const uint32_t b = __float_as_uint(v + 0.0f);
+  return b ^ ((int32_t)b < 0 ? 0xffffffffu : 0x80000000u);
+}
+
 // Top-k of a row held as v[j] <-> element lane + 32*j (elements >= n are not candidates).
-// Lane j (< k) returns the j-th result in (rv, ri).
+// Lane j (< k) returns the j-th result in (rv, ri).  Every round is a scan of the lane's registers and two warp
+// reductions (largest key, then the lowest index that has it): an argmax by shuffles is five dependent steps of two
+// shuffles each, and k rounds of it were most of this kernel's time (with the divisions of group_mask: 256 experts in 8
+// groups, 64 tokens 14.7 -> 7.8 us, 2048 tokens 18.7 -> 10.0 us).
 template <int VPT>
 __device__ __forceinline__ void warp_topk(const float (&v)[VPT], int n, int k, int lane, float& rv,
                                           int& ri) {
-  uint32_t taken = 0;
+  uint32_t key[VPT];  // 0 = no candidate (below every key: the key of -inf is 0x007fffff)
+#pragma unroll
+  for (int j = 0; j < VPT; ++j) key[j] = lane + 32 * j < n ? order_key(v[j]) : 0u;
   rv = -INFINITY;
   ri = 0;
   for (int it = 0; it < k; ++it) {
+    uint32_t bk = 0;
     float bv = -INFINITY;
     int bi = INT_MAX;
 #pragma unroll
-    for (int j = 0; j < VPT; ++j) {
-      int e = lane + 32 * j;
-      bool cand = e < n && !((taken >> j) & 1u);
-      if (cand && (bi == INT_MAX || v[j] > bv)) {  // ascending e inside a lane: first max wins
-        bv = v[j];
-        bi = e;
-      }
-    }
-    warp_argmax(bv, bi);
-    if (bi != INT_MAX && (bi & 31) == lane) taken |= 1u << (bi >> 5);
-    if (lane == it) {
-      rv = bv;
-      ri = bi == INT_MAX ? 0 : bi;
-    }
+    for (int j = 0; j < VPT; ++j)
+      if (key[j] > bk) bk = key[j], bv = v[j], bi = lane + 32 * j;  // ascending inside a lane: the first maximum wins
+    const uint32_t best = __reduce_max_sync(0xffffffffu, bk);
+    const int idx = (int)__reduce_min_sync(0xffffffffu, bk == best ? (uint32_t)bi : (uint32_t)INT_MAX);
+    if (idx == INT_MAX) break;  // (uniform) no candidate left
+    bv = __shfl_sync(0xffffffffu, bv, idx & 31);
+#pragma unroll
+    for (int j = 0; j < VPT; ++j)
+      if (lane + 32 * j == idx) key[j] = 0u;
+    if (lane == it) rv = bv, ri = idx;
   }
 }
 
@@ -61,13 +70,18 @@ template <int VPT>
 __device__ __forceinline__ void group_mask(float (&v)[VPT], int n, int n_groups, int topk_groups,
                                            int dtype, int lane) {
   const int gsz = n / n_groups;
+  // e / gsz for e < 1024 as a multiplication (the error of the rounded-up reciprocal stays below 1023 / 2^20 < 1 / gsz),
+  // once per element: a division per element and group was most of the time of a grouped selection
+  const uint32_t inv = ((1u << 20) + gsz - 1) / gsz;
+  int grp[VPT];
+#pragma unroll
+  for (int j = 0; j < VPT; ++j) grp[j] = lane + 32 * j < n ? (int)(((uint32_t)(lane + 32 * j) * inv) >> 20) : -1;
   float my_gs = -INFINITY;  // lane g holds the score of group g
   for (int g = 0; g < n_groups; ++g) {
     float a1 = -INFINITY, a2 = -INFINITY;
 #pragma unroll
     for (int j = 0; j < VPT; ++j) {
-      int e = lane + 32 * j;
-      if (e < n && e / gsz == g) {
+      if (grp[j] == g) {
         float x = v[j];
         if (x > a1) {
           a2 = a1;
@@ -101,10 +115,8 @@ __device__ __forceinline__ void group_mask(float (&v)[VPT], int n, int n_groups,
     }
   }
 #pragma unroll
-  for (int j = 0; j < VPT; ++j) {
-    int e = lane + 32 * j;
-    if (e < n && !((keep >> (e / gsz)) & 1u)) v[j] = -INFINITY;
-  }
+  for (int j = 0; j < VPT; ++j)
+    if (grp[j] >= 0 && !((keep >> grp[j]) & 1u)) v[j] = -INFINITY;
 }
 
 template <int VPT>
@@ -200,15 +212,31 @@ route_kernel(int32_t* __restrict__ ids, float* __restrict__ w, __nv_bfloat16* __
 
 // ---- router GEMM ---------------------------------------------------------------------------------
 // logits[t,e] = sum_h x[t,h] * wr[e,h]; bf16 operands, fp32 accumulation on the warp-level tensor path
-// (mma.sync m16n8k16).  It is ~0.5 % of the layer's FLOPs, so it stays a small, plain kernel: CTA tile
-// 32 tokens x 64 experts, K chunks of 64 staged in shared memory, 4 warps each owning 16 token rows x 32 experts.
-constexpr int RG_BM = 32, RG_BN = 64, RG_BK = 64, RG_LD = RG_BK + 8, RG_STAGES = 3;  // +8 bf16: conflict-free fragment reads
+// (mma.sync m16n8k16).  It is ~0.5 % of the layer's FLOPs and bound by the copies of x and wr on their way to shared
+// memory, so what counts is how many of them are in flight: a block owns 64 tokens x 128 experts (x is read once up to
+// 128 experts), four stages of 64 K columns, and when that leaves SMs without a block the K range is split over the
+// blocks of a cluster, which add their tiles up through distributed shared memory, in rank order (the result does not
+// depend on timing).  Measured against 32 x 64 tiles that walk all of K (64 tokens of the DeepSeek shape were 8 blocks
+// with 112 dependent steps each): 42 -> 15 us there, 57 -> 43 us at 2048 tokens,
+// 34 -> 25 us for 8192 tokens of the Qwen3 shape.
+constexpr int RG_BM = 64, RG_BN = 128, RG_BK = 64, RG_LD = RG_BK + 8, RG_STAGES = 4;  // +8 bf16: conflict-free ldmatrix
+constexpr int RG_THREADS = 256;
+constexpr int RG_STAGE_ELEMS = (RG_BM + RG_BN) * RG_LD;
+constexpr size_t RG_SMEM_BYTES = (size_t)RG_STAGES * RG_STAGE_ELEMS * sizeof(__nv_bfloat16);
+constexpr int RG_CLD = RG_BN + 4;  // fp32 tile on its way between the blocks of a cluster
+static_assert((size_t)RG_BM * RG_CLD * sizeof(float) <= RG_SMEM_BYTES, "the fp32 tile reuses the stages");
+constexpr int RG_MAX_SPLIT = 8;  // portable cluster size
 
-__device__ __forceinline__ void mma_bf16_16816(float (&d)[4], const uint32_t (&a)[4], const uint32_t (&b)[2]) {
+__device__ __forceinline__ void mma_bf16_16816(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
   asm volatile(
       "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
       : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ void ldmatrix_x4(uint32_t (&r)[4], const void* p) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"((uint32_t)__cvta_generic_to_shared(p)));
 }
 
 // 16-byte asynchronous copy global -> shared; bytes = 0 writes zeros (rows / columns past the end)
@@ -218,85 +246,114 @@ __device__ __forceinline__ void cp_async16(void* smem_dst, const void* gsrc, int
                : "memory");
 }
 
-__global__ void __launch_bounds__(128)
+// grid (ceil(T / 64), splits, ceil(E / 128)), clusters of (1, splits, 1)
+__global__ void __launch_bounds__(RG_THREADS)
 router_gemm_kernel(float* __restrict__ logits, const __nv_bfloat16* __restrict__ x,
                    const __nv_bfloat16* __restrict__ wr, int64_t T, int64_t H, int64_t E) {
-  // Three stages: the copies of K chunks kt+1 and kt+2 are in flight while the MMAs of chunk kt run.  The MMAs of a
-  // chunk are a few hundred cycles and a copy is an L2 round trip, so the kernel lives on copies in flight: tiles
-  // of 32 rows (twice the blocks of a 64-row tile, two or three per SM) and three stages keep about four chunks
-  // per SM on their way.  A sum over K is formed in the same order whatever the tiling: logits do not change.
-  __shared__ __align__(16) __nv_bfloat16 sA[RG_STAGES][RG_BM * RG_LD];
-  __shared__ __align__(16) __nv_bfloat16 sB[RG_STAGES][RG_BN * RG_LD];
+  extern __shared__ __align__(16) uint8_t rg_smem[];
+  __nv_bfloat16* const stages = reinterpret_cast<__nv_bfloat16*>(rg_smem);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int wm = warp & 1, wn = warp >> 1;  // the warp's 16 rows and 32 columns of the 32 x 64 tile
-  const int64_t t0 = (int64_t)blockIdx.x * RG_BM, e0 = (int64_t)blockIdx.y * RG_BN;
-  float acc[4][4];
+  const int wm = warp & 1, wn = warp >> 1;  // the warp's 32 rows and 32 columns of the 64 x 128 tile
+  const int splits = gridDim.y, rank = blockIdx.y;
+  const int64_t t0 = (int64_t)blockIdx.x * RG_BM, e0 = (int64_t)blockIdx.z * RG_BN;
+  const int nk = (int)((H + RG_BK - 1) / RG_BK);
+  const int k_begin = (int)((int64_t)nk * rank / splits), k_end = (int)((int64_t)nk * (rank + 1) / splits);
+  float acc[2][4][4];
 #pragma unroll
-  for (int i = 0; i < 4; ++i)
+  for (int m = 0; m < 2; ++m)
 #pragma unroll
-    for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
-  const int g = lane >> 2, tq = lane & 3;
-  auto load_stage = [&](int st, int64_t k0) {
-    // A: 32 rows x 64 bf16 = 256 chunks of 16 B (128 threads x 2); B: 64 rows = 512 chunks (x 4)
+    for (int i = 0; i < 4; ++i)
 #pragma unroll
-    for (int i = 0; i < 2; ++i) {
-      const int c = tid + i * 128;
+      for (int j = 0; j < 4; ++j) acc[m][i][j] = 0.f;
+  auto load_stage = [&](int kt) {
+    __nv_bfloat16* const st = stages + (size_t)((kt - k_begin) % RG_STAGES) * RG_STAGE_ELEMS;
+    const int64_t k0 = (int64_t)kt * RG_BK;
+#pragma unroll
+    for (int i = 0; i < (RG_BM + RG_BN) * 8 / RG_THREADS; ++i) {  // rows of x, then rows of wr; 8 chunks of 16 B each
+      const int c = tid + i * RG_THREADS;
       const int r = c >> 3, cc = (c & 7) * 8;
-      const bool ok = k0 + cc < H && t0 + r < T;
-      cp_async16(sA[st] + r * RG_LD + cc, ok ? x + (t0 + r) * H + k0 + cc : x, ok ? 16 : 0);
-    }
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int c = tid + i * 128;
-      const int r = c >> 3, cc = (c & 7) * 8;
-      const bool ok = k0 + cc < H && e0 + r < E;
-      cp_async16(sB[st] + r * RG_LD + cc, ok ? wr + (e0 + r) * H + k0 + cc : wr, ok ? 16 : 0);
+      const bool is_x = r < RG_BM;
+      const int64_t row = is_x ? t0 + r : e0 + r - RG_BM;
+      const bool on = k0 + cc < H && row < (is_x ? T : E);
+      const __nv_bfloat16* src = (is_x ? x : wr) + (on ? row * H + k0 + cc : 0);
+      cp_async16(st + r * RG_LD + cc, src, on ? 16 : 0);
     }
   };
-  const int nk = (int)((H + RG_BK - 1) / RG_BK);
-  // one commit group per chunk, empty where there is no chunk left, so that "all but the two newest groups are
-  // complete" always means "chunk kt has landed"
-  load_stage(0, 0);
-  asm volatile("cp.async.commit_group;" ::: "memory");
-  if (nk > 1) load_stage(1, RG_BK);
-  asm volatile("cp.async.commit_group;" ::: "memory");
-  for (int kt = 0; kt < nk; ++kt) {
-    const int st = kt % RG_STAGES;
-    if (kt + 2 < nk) load_stage((kt + 2) % RG_STAGES, (int64_t)(kt + 2) * RG_BK);
+  // one commit group per chunk, empty where there is no chunk left, so that "all but the newest groups are complete"
+  // always means "chunk kt has landed"
+#pragma unroll
+  for (int s = 0; s < RG_STAGES - 1; ++s) {
+    if (k_begin + s < k_end) load_stage(k_begin + s);
     asm volatile("cp.async.commit_group;" ::: "memory");
-    asm volatile("cp.async.wait_group 2;" ::: "memory");
-    __syncthreads();
+  }
+  for (int kt = k_begin; kt < k_end; ++kt) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(RG_STAGES - 2) : "memory");
+    __syncthreads();  // chunk kt is there for everyone, and everyone is done with the stage that is filled next
+    if (kt + RG_STAGES - 1 < k_end) load_stage(kt + RG_STAGES - 1);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    const __nv_bfloat16* sA = stages + (size_t)((kt - k_begin) % RG_STAGES) * RG_STAGE_ELEMS;
+    const __nv_bfloat16* sB = sA + RG_BM * RG_LD;
 #pragma unroll
     for (int kk = 0; kk < RG_BK; kk += 16) {
-      uint32_t a[4];
-      const __nv_bfloat16* pa = sA[st] + (wm * 16 + g) * RG_LD + kk + tq * 2;
-      a[0] = *reinterpret_cast<const uint32_t*>(pa);
-      a[1] = *reinterpret_cast<const uint32_t*>(pa + 8 * RG_LD);
-      a[2] = *reinterpret_cast<const uint32_t*>(pa + 8);
-      a[3] = *reinterpret_cast<const uint32_t*>(pa + 8 * RG_LD + 8);
+      uint32_t a[2][4], b[2][4];
 #pragma unroll
-      for (int nb = 0; nb < 4; ++nb) {
-        uint32_t b[2];
-        const __nv_bfloat16* pb = sB[st] + (wn * 32 + nb * 8 + g) * RG_LD + kk + tq * 2;
-        b[0] = *reinterpret_cast<const uint32_t*>(pb);
-        b[1] = *reinterpret_cast<const uint32_t*>(pb + 8);
-        mma_bf16_16816(acc[nb], a, b);
-      }
-    }
-    __syncthreads();  // the stage is overwritten by the copies issued at the top of the next iteration
-  }
+      for (int m = 0; m < 2; ++m)  // rows 0-7 / 8-15 at k, then the same at k + 8
+        ldmatrix_x4(a[m], sA + (wm * 32 + m * 16 + (lane & 15)) * RG_LD + kk + (lane >> 4) * 8);
 #pragma unroll
-  for (int nb = 0; nb < 4; ++nb) {
-    int64_t r0 = t0 + wm * 16 + g, c0 = e0 + wn * 32 + nb * 8 + tq * 2;
-    if (r0 < T) {
-      if (c0 < E) logits[r0 * E + c0] = acc[nb][0];
-      if (c0 + 1 < E) logits[r0 * E + c0 + 1] = acc[nb][1];
-    }
-    if (r0 + 8 < T) {
-      if (c0 < E) logits[(r0 + 8) * E + c0] = acc[nb][2];
-      if (c0 + 1 < E) logits[(r0 + 8) * E + c0 + 1] = acc[nb][3];
+      for (int p = 0; p < 2; ++p)  // columns 0-7 at k, k + 8, then columns 8-15
+        ldmatrix_x4(b[p], sB + (wn * 32 + p * 16 + (lane & 7) + ((lane >> 4) << 3)) * RG_LD + kk + ((lane >> 3) & 1) * 8);
+#pragma unroll
+      for (int m = 0; m < 2; ++m)
+#pragma unroll
+        for (int nb = 0; nb < 4; ++nb) mma_bf16_16816(acc[m][nb], a[m], b[nb >> 1][(nb & 1) * 2], b[nb >> 1][(nb & 1) * 2 + 1]);
     }
   }
+  const int g = lane >> 2, tq = lane & 3;
+  if (splits == 1) {
+#pragma unroll
+    for (int m = 0; m < 2; ++m)
+#pragma unroll
+      for (int nb = 0; nb < 4; ++nb)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const int64_t r = t0 + wm * 32 + m * 16 + g + (i >> 1) * 8, c = e0 + wn * 32 + nb * 8 + tq * 2 + (i & 1);
+          if (r < T && c < E) logits[r * E + c] = acc[m][nb][i];
+        }
+    return;
+  }
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+  __syncthreads();  // the stages are free: the tile goes there
+  float* const tile = reinterpret_cast<float*>(rg_smem);
+#pragma unroll
+  for (int m = 0; m < 2; ++m)
+#pragma unroll
+    for (int nb = 0; nb < 4; ++nb)
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        tile[(wm * 32 + m * 16 + g + (i >> 1) * 8) * RG_CLD + wn * 32 + nb * 8 + tq * 2 + (i & 1)] = acc[m][nb][i];
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+  // every block sums and stores its share of the tile's rows
+  const uint32_t tile_addr = (uint32_t)__cvta_generic_to_shared(tile);
+  const int rows = RG_BM / splits;
+  for (int i = tid; i < rows * (RG_BN / 4); i += RG_THREADS) {
+    const int r = rank * rows + i / (RG_BN / 4), c = (i % (RG_BN / 4)) * 4;
+    float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int p = 0; p < splits; ++p) {
+      uint32_t addr;
+      float4 v;
+      asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(addr) : "r"(tile_addr + (uint32_t)(r * RG_CLD + c) * 4u), "r"(p));
+      asm volatile("ld.shared::cluster.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
+      sum.x += v.x, sum.y += v.y, sum.z += v.z, sum.w += v.w;
+    }
+    if (t0 + r < T) {
+      float* dst = logits + (t0 + r) * E + e0 + c;
+      const float s4[4] = {sum.x, sum.y, sum.z, sum.w};
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (e0 + c + u < E) dst[u] = s4[u];
+    }
+  }
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");  // no block leaves while its tile is read
 }
 
 // Small-T variant (decode): one block per expert row; its 4 warps split H (16-byte loads) and dot the slice with up
@@ -488,8 +545,30 @@ extern "C" int b200moe_router_logits(float* logits, const void* x, const void* w
     if (E <= 8) router_small_e_kernel<8><<<grid, RS_WARPS * 32, 0, (cudaStream_t)stream>>>(logits, xb, wb, T, H, (int)E);
     else router_small_e_kernel<16><<<grid, RS_WARPS * 32, 0, (cudaStream_t)stream>>>(logits, xb, wb, T, H, (int)E);
   } else {
-    dim3 grid((unsigned)((T + RG_BM - 1) / RG_BM), (unsigned)((E + RG_BN - 1) / RG_BN));
-    router_gemm_kernel<<<grid, 128, 0, (cudaStream_t)stream>>>(logits, xb, wb, T, H, E);
+    constexpr int kMaxDevices = 64;
+    static bool attr_done[kMaxDevices] = {};
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return B200MOE_EDRIVER;
+    if (!attr_done[dev]) {  // per-device attribute
+      cudaFuncSetAttribute(router_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)RG_SMEM_BYTES);
+      attr_done[dev] = true;
+    }
+    const int64_t mt = (T + RG_BM - 1) / RG_BM, nt = (E + RG_BN - 1) / RG_BN;
+    int splits = 1;  // as many as there are SMs for, with at least 256 columns of K each
+    while (splits < RG_MAX_SPLIT && mt * nt * splits * 2 <= moe_device_sm_count() && H / (splits * 2) >= 4 * RG_BK) splits *= 2;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)mt, (unsigned)splits, (unsigned)nt);
+    cfg.blockDim = dim3(RG_THREADS);
+    cfg.dynamicSmemBytes = RG_SMEM_BYTES;
+    cfg.stream = (cudaStream_t)stream;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = at[0].val.clusterDim.z = 1;
+    at[0].val.clusterDim.y = (unsigned)splits;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, router_gemm_kernel, logits, xb, wb, T, H, E);
+    if (e != cudaSuccess) return (int)e;
   }
   return moe_launch_status();
 }
