@@ -39,7 +39,7 @@ def _run(cmd, verbose):
 
 def build_native(force=False, verbose=False):
     srcs = [os.path.join(CSRC, s) for s in CU_SOURCES]
-    deps = srcs + [os.path.join(CSRC, h) for h in ("common.cuh", "internal.h", "tc_ptx.cuh")] + [
+    deps = srcs + [os.path.join(CSRC, h) for h in ("common.cuh", "internal.h", "schedule.h", "tc_ptx.cuh")] + [
         os.path.join(ROOT, "include", "b200moe.h")]
     if not force and not _newer(NATIVE_LIB, deps):
         return NATIVE_LIB

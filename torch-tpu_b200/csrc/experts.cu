@@ -33,7 +33,7 @@ int choose_ksplit(int64_t P, int64_t E, int64_t H, int64_t I) {
 }
 
 struct WsLayout {
-  size_t offsets, sorted, pos_of, scratch, mtiles, nmt, xq, xs, hq, hs, y, sc32, s_sc32, y32, s_y32, acc32;
+  size_t offsets, sorted, pos_of, scratch, mtiles, nmt, xq, xs, hq, hs, y, sc32, s_sc32, y32, s_y32, acc32, part, cnt, s_part, s_cnt;
   size_t s_offsets, s_mtiles, s_nmt, s_xq, s_xs, s_hq, s_hs, s_y;
   size_t total;
   int64_t P, ld, lds;
@@ -79,6 +79,9 @@ WsLayout make_layout(const b200moe_experts_desc& d) {
   // fp32 partial sums of the K-split down GEMM (decode-size batches only)
   // (sized for min(P, limit) rows whatever P is, so that the workspace size never shrinks when T grows)
   L.y32 = take(w8a8 ? (size_t)(P < kSplitMaxPairs ? P : kSplitMaxPairs) * d.H * sizeof(float) : 0);
+  // partial sums and counters of tiles that CTAs share
+  L.part = take(w8a8 ? moe_split_part_bytes(P) : 0);
+  L.cnt = take(kSplitCounters * sizeof(int32_t));
   // fp32 copies of bf16 block scales (the tensor-core kernels read fp32 scales only)
   L.sc32 = take(d.scale_dtype == B200MOE_BF16 && w8a8 ? 3 * (size_t)d.E * nI * nH * sizeof(float) : 0);
   if (d.I_shared > 0) {
@@ -92,6 +95,8 @@ WsLayout make_layout(const b200moe_experts_desc& d) {
     L.s_hs = take(w8a8 ? nIs * (size_t)L.lds * sizeof(float) : 0);
     L.s_y = take((size_t)d.T * d.H * 2);
     L.s_y32 = take(w8a8 ? (size_t)(d.T < kSplitMaxPairs ? d.T : kSplitMaxPairs) * d.H * sizeof(float) : 0);
+    L.s_part = take(w8a8 ? moe_split_part_bytes(d.T) : 0);
+    L.s_cnt = take(kSplitCounters * sizeof(int32_t));
     L.s_sc32 = take(d.scale_dtype == B200MOE_BF16 && w8a8 ? 3 * nIs * nH * sizeof(float) : 0);
   }
   L.total = o;
@@ -226,10 +231,10 @@ extern "C" int b200moe_experts(void* out, const void* x, const void* w_gate, con
   if (do_prep) {
     bool tiles_done = false;
     rc = moe_permute_impl(I32(L.sorted), I32(L.offsets), ids, d->T, d->k, d->E, I32(L.scratch), status, I32(L.pos_of),
-                          I32(L.mtiles), I32(L.nmt), L.max_mtiles, &tiles_done, stream);
+                          I32(L.mtiles), I32(L.nmt), L.max_mtiles, I32(L.cnt), &tiles_done, stream);
     if (rc) return rc;
     if (!tiles_done) {
-      rc = moe_build_mtiles(I32(L.mtiles), I32(L.nmt), I32(L.offsets), (int)d->E, L.P, L.max_mtiles, st);
+      rc = moe_build_mtiles(I32(L.mtiles), I32(L.nmt), I32(L.offsets), (int)d->E, L.P, L.max_mtiles, I32(L.cnt), st);
       if (rc) return rc;
     }
   }
@@ -275,6 +280,7 @@ extern "C" int b200moe_experts(void* out, const void* x, const void* w_gate, con
   g.hq = reinterpret_cast<uint8_t*>(ws + L.hq);
   g.hs_t = reinterpret_cast<float*>(ws + L.hs);
   g.h16 = reinterpret_cast<__nv_bfloat16*>(ws + L.hq);
+  if (w8a8) g.split = MoeSplitBuffers{reinterpret_cast<float*>(ws + L.part), I32(L.cnt)};
   g.status = status;
   __nv_bfloat16* xg = reinterpret_cast<__nv_bfloat16*>(ws + L.xq);  // W8A16 tensor-core path: x rows in sorted order
   if (tc1_16 && do_prep) {
@@ -332,7 +338,7 @@ extern "C" int b200moe_experts(void* out, const void* x, const void* w_gate, con
   if (d->I_shared > 0) {
     cudaStream_t ss = side ? side->s : st;
     if (do_prep) {
-      const MoeIdentityLists lists{I32(L.s_offsets), I32(L.s_mtiles), I32(L.s_nmt)};
+      const MoeIdentityLists lists{I32(L.s_offsets), I32(L.s_mtiles), I32(L.s_nmt), I32(L.s_cnt)};
       rc = w8a8 ? moe_quant_identity(reinterpret_cast<uint8_t*>(ws + L.s_xq), reinterpret_cast<float*>(ws + L.s_xs),
                                      L.lds, x, d->T, d->H, lists, ss)
                 : moe_identity_lists(lists, d->T, ss);
@@ -366,6 +372,7 @@ extern "C" int b200moe_experts(void* out, const void* x, const void* w_gate, con
     s.P = d->T;
     s.I = (int)d->I_shared;
     s.E = 1;
+    if (w8a8) s.split = MoeSplitBuffers{reinterpret_cast<float*>(ws + L.s_part), I32(L.s_cnt)};
     s.hq = reinterpret_cast<uint8_t*>(ws + L.s_hq);
     s.hs_t = reinterpret_cast<float*>(ws + L.s_hs);
     s.h16 = reinterpret_cast<__nv_bfloat16*>(ws + L.s_hq);
@@ -485,7 +492,7 @@ int grouped_mlp_impl(void* y, const uint8_t* xq, const float* xs_t, int64_t ld, 
   if (row_src && !use_tc) return B200MOE_EDRIVER;  // peer output exists on the tensor-core path only
   int32_t* mtiles = reinterpret_cast<int32_t*>(ws + L.mtiles);
   int32_t* nmt = reinterpret_cast<int32_t*>(ws + L.nmt);
-  int rc = moe_build_mtiles(mtiles, nmt, expert_offsets, (int)E, R, L.max_mtiles, st);
+  int rc = moe_build_mtiles(mtiles, nmt, expert_offsets, (int)E, R, L.max_mtiles, nullptr, st);
   if (rc) return rc;
   const void *sg = s_gate, *su = s_up, *sd = s_down;
   int sdt = scale_dtype;
@@ -563,7 +570,7 @@ extern "C" int b200moe_grouped_mlp_remote(const uint64_t* out_tbl, const int32_t
 // ---- plain FP8 block-scaled linear layer -----------------------------------------------------------------
 namespace {
 struct LinLayout {
-  size_t offsets, mtiles, nmt, xq, xs, sc32, total;
+  size_t offsets, mtiles, nmt, xq, xs, sc32, part, cnt, total;
   int64_t ld;
   int max_mtiles;
 };
@@ -584,6 +591,8 @@ LinLayout lin_layout(int64_t M, int64_t K, int64_t N, int scale_dtype) {
   L.xq = take((size_t)L.ld * K);
   L.xs = take((size_t)(K / kBlock) * L.ld * sizeof(float));
   L.sc32 = take(scale_dtype == B200MOE_BF16 ? (size_t)((N + kBlock - 1) / kBlock) * (K / kBlock) * sizeof(float) : 0);
+  L.part = take(moe_split_part_bytes(M));
+  L.cnt = take(kSplitCounters * sizeof(int32_t));
   L.total = o;
   return L;
 }
@@ -616,8 +625,9 @@ extern "C" int b200moe_linear_w8(void* out, const void* x, const void* w, const 
   int32_t* offsets = reinterpret_cast<int32_t*>(ws + L.offsets);
   int32_t* mtiles = reinterpret_cast<int32_t*>(ws + L.mtiles);
   int32_t* nmt = reinterpret_cast<int32_t*>(ws + L.nmt);
+  int32_t* cnt = reinterpret_cast<int32_t*>(ws + L.cnt);
   int rc = moe_quant_identity(reinterpret_cast<uint8_t*>(ws + L.xq), reinterpret_cast<float*>(ws + L.xs), L.ld, x, M, K,
-                              MoeIdentityLists{offsets, mtiles, nmt}, st);
+                              MoeIdentityLists{offsets, mtiles, nmt, cnt}, st);
   if (rc) return rc;
   const void* sc = scale;
   if (scale_dtype == B200MOE_BF16) {
@@ -644,6 +654,7 @@ extern "C" int b200moe_linear_w8(void* out, const void* x, const void* w, const 
   g.H = (int)K;
   g.I = (int)N;
   g.E = 1;
+  g.split = MoeSplitBuffers{reinterpret_cast<float*>(ws + L.part), cnt};
   g.out = reinterpret_cast<__nv_bfloat16*>(out);
   g.status = status;
   return moe_linear_tc(g, st);
@@ -656,7 +667,7 @@ __global__ void fill_scalar_scale_kernel(float* __restrict__ dst, const float* _
   if (i < n) dst[i] = scale ? *scale : 1.0f;
 }
 struct SmmLayout {
-  size_t offsets, mtiles, nmt, xs, ws, total;
+  size_t offsets, mtiles, nmt, xs, ws, part, cnt, total;
   int64_t ld;
   int max_mtiles;
 };
@@ -676,6 +687,8 @@ SmmLayout smm_layout(int64_t M, int64_t K, int64_t N) {
   L.nmt = take(sizeof(int32_t));
   L.xs = take((size_t)(K / kBlock) * L.ld * sizeof(float));
   L.ws = take((size_t)((N + kBlock - 1) / kBlock) * (K / kBlock) * sizeof(float));
+  L.part = take(moe_split_part_bytes(M));
+  L.cnt = take(kSplitCounters * sizeof(int32_t));
   L.total = o;
   return L;
 }
@@ -704,7 +717,8 @@ extern "C" int b200moe_scaled_mm(void* out, int out_dtype, const void* a, const 
   int32_t* offsets = reinterpret_cast<int32_t*>(ws + L.offsets);
   int32_t* mtiles = reinterpret_cast<int32_t*>(ws + L.mtiles);
   int32_t* nmt = reinterpret_cast<int32_t*>(ws + L.nmt);
-  int rc = moe_identity_lists(MoeIdentityLists{offsets, mtiles, nmt}, M, st);
+  int32_t* cnt = reinterpret_cast<int32_t*>(ws + L.cnt);
+  int rc = moe_identity_lists(MoeIdentityLists{offsets, mtiles, nmt, cnt}, M, st);
   if (rc) return rc;
   // the kernel applies act_scale[row,kb] * weight_scale[nb,kb] to every 128-deep partial sum: constant grids here
   const int64_t nxs = (K / kBlock) * L.ld, nws = ((N + kBlock - 1) / kBlock) * (K / kBlock);
@@ -728,6 +742,7 @@ extern "C" int b200moe_scaled_mm(void* out, int out_dtype, const void* a, const 
   g.H = (int)K;
   g.I = (int)N;
   g.E = 1;
+  g.split = MoeSplitBuffers{reinterpret_cast<float*>(ws + L.part), cnt};
   if (out_dtype == B200MOE_F32) g.out32 = reinterpret_cast<float*>(out);
   else g.out = reinterpret_cast<__nv_bfloat16*>(out);
   g.status = status;

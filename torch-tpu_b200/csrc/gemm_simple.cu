@@ -200,7 +200,8 @@ __global__ void __launch_bounds__(256) gemm2_simple_kernel(MoeGemmArgs a) {
 
 __global__ void __launch_bounds__(1024)
 build_mtiles_kernel(int32_t* __restrict__ mtiles, int32_t* __restrict__ num_mtiles,
-                    const int32_t* __restrict__ offsets, int E, int max_rows, int max_mtiles) {
+                    const int32_t* __restrict__ offsets, int E, int max_rows, int max_mtiles, int32_t* split_cnt) {
+  moe_clear_counters(split_cnt);
   __shared__ int tmp[1024];
   const int t = threadIdx.x;
   int b = 0, n = 0;
@@ -295,8 +296,8 @@ combine_kernel(__nv_bfloat16* __restrict__ out, const __nv_bfloat16* __restrict_
 }  // namespace
 
 int moe_build_mtiles(int32_t* mtiles, int32_t* num_mtiles, const int32_t* offsets, int E, int64_t max_rows,
-                     int max_mtiles, cudaStream_t st) {
-  build_mtiles_kernel<<<1, 1024, 0, st>>>(mtiles, num_mtiles, offsets, E, (int)max_rows, max_mtiles);
+                     int max_mtiles, int32_t* split_cnt, cudaStream_t st) {
+  build_mtiles_kernel<<<1, 1024, 0, st>>>(mtiles, num_mtiles, offsets, E, (int)max_rows, max_mtiles, split_cnt);
   return moe_launch_status();
 }
 

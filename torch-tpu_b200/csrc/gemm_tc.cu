@@ -22,6 +22,7 @@
 //
 // No multicast loads anywhere.  Every wait is bounded: on a time-out the CTA raises status bit 1, all roles
 // leave their loops, tensor memory is released and the kernel returns.
+#include "schedule.h"
 #include "tc_ptx.cuh"
 
 namespace {
@@ -62,6 +63,7 @@ struct TcShared {
   uint64_t dst_full, dst_empty;    // same for the destinations of the item's result rows (taken at the item's END)
   uint32_t tmem_base;
   int abort_flag;
+  int part_last;           // this CTA left the last part of a shared tile: it finishes the tile
   int head_item[8];        // expert, first row, end of the expert's rows, n-tile, first K block, K blocks
   float head_w[4];         // weight scales of the item's first two K blocks: (gate|half 0, up|half 1) x 2
   float head_sa[2][128];   // activation scales of the first two K blocks, per row of the tile
@@ -88,6 +90,11 @@ struct TcArgs {
   int H, I, NT;
   int P;         // rows the operand buffers hold: row ranges are clipped to it
   int KS;        // K splits (down GEMM of decode-size batches); 1 = none
+  // down GEMM / linear layer: tiles of a nearly empty last round are shared between CTAs (schedule.h); one slot of partial
+  // sums (part_slot floats) per CTA and one counter per shared tile, zero between launches.  NULL = tiles stay whole
+  float* part;
+  int32_t* part_cnt;
+  int part_slot, part_rows;
   int m_major;   // work-item order: 0 = n-tile slow, m-tile fast; 1 = m-tile slow, n-tile fast (see launch_tc)
   float* out32;  // fp32 accumulation target when KS > 1; with KS == 1 (linear layer only): fp32 rows stored instead of bf16
   // down GEMM with the weighted combine fused in: row r adds comb_w[pair] * y[r,:] into comb32[pair / div, :] (fp32,
@@ -168,8 +175,11 @@ moe_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
   const uint32_t tmem_base = sh->tmem_base;
 
   const int num_mtiles = *a.num_mtiles;
-  const int total_tiles = num_mtiles * a.NT * a.KS;  // work items: (n-tile, m-tile, K split)
   const int KB_all = (GEMM2 ? a.I : a.H) / kBlock;
+  // work items: (n-tile, m-tile, K split); without a K split the last ones may be parts of shared tiles
+  WorkPlan plan{num_mtiles * a.NT * a.KS, 1, num_mtiles * a.NT * a.KS, KB_all};
+  if (MODE != 0 && a.part) plan = work_plan(num_mtiles * a.NT, KB_all, gridDim.x, a.part_rows);
+  const int total_tiles = plan.items;
   const int nH = a.H / kBlock, nI = a.I / kBlock;
 
   // weight-scale addressing: gemm1 s[e, nt, kb] (gate, up); gemm2 s[e, kb, 2*nt + j]; scales are fp32 here.
@@ -184,9 +194,16 @@ moe_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
   };
   auto item_of = [&](int t) {
     Item w;
-    const int ks = t % a.KS, tt = t / a.KS;
+    int ks = 0, tt = t;
+    if (MODE != 0 && a.part) {
+      const WorkItem i = work_item(plan, t);
+      tt = i.tile, w.kb0 = i.kb0, w.KB = i.KB;
+    } else {
+      ks = t % a.KS, tt = t / a.KS;
+    }
     w.nt = a.m_major ? tt % a.NT : tt / num_mtiles;
     w.mt = a.m_major ? tt / a.NT : tt - w.nt * num_mtiles;
+    if (MODE != 0 && a.part) return w;
     w.kb0 = (int)((int64_t)KB_all * ks / a.KS);
     w.KB = (int)((int64_t)KB_all * (ks + 1) / a.KS) - w.kb0;  // K blocks of this work item
     return w;
@@ -206,21 +223,19 @@ moe_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
       bool ok = true;
       // the m-tile list entry of the NEXT work item is requested while this one's loads are issued: when the weights
       // stream from HBM the ring is empty at every tile start, and a dependent L2 round trip there is pure idle time
-      auto mtile_of = [&](int t) {
-        const int tt = t / a.KS;
-        return a.m_major ? tt / a.NT : tt % num_mtiles;
-      };
+      Item nx{};
       int nx_e = 0, nx_row0 = 0;
-      if ((int)blockIdx.x < total_tiles) nx_e = a.mtiles[2 * mtile_of(blockIdx.x)], nx_row0 = a.mtiles[2 * mtile_of(blockIdx.x) + 1];
+      if ((int)blockIdx.x < total_tiles) {
+        nx = item_of(blockIdx.x);
+        nx_e = a.mtiles[2 * nx.mt], nx_row0 = a.mtiles[2 * nx.mt + 1];
+      }
       for (int t = blockIdx.x; t < total_tiles && ok; t += gridDim.x) {
-        const int ks = t % a.KS, tt = t / a.KS;
-        const int nt = a.m_major ? tt % a.NT : tt / num_mtiles;
+        const int nt = nx.nt, kb0 = nx.kb0, kb1 = nx.kb0 + nx.KB;
         const int e = nx_e, row0 = nx_row0;
         if (t + (int)gridDim.x < total_tiles) {
-          const int mn = mtile_of(t + gridDim.x);
-          nx_e = a.mtiles[2 * mn], nx_row0 = a.mtiles[2 * mn + 1];
+          nx = item_of(t + gridDim.x);
+          nx_e = a.mtiles[2 * nx.mt], nx_row0 = a.mtiles[2 * nx.mt + 1];
         }
-        const int kb0 = (int)((int64_t)KB_all * ks / a.KS), kb1 = (int)((int64_t)KB_all * (ks + 1) / a.KS);
         for (int kb = kb0; kb < kb1; ++kb, ++it) {
           const int s = it % TC_STAGES;
           const uint32_t ph = (it / TC_STAGES) & 1;
@@ -256,8 +271,12 @@ moe_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
                                     : make_smem_desc(smem_base + TC_A_BYTES, 16, 1024);
       uint32_t n_it = 0;
       for (int t = blockIdx.x; t < total_tiles; t += gridDim.x) {
-        const int ks = t % a.KS;
-        n_it += (uint32_t)((int)((int64_t)KB_all * (ks + 1) / a.KS) - (int)((int64_t)KB_all * ks / a.KS));
+        if (MODE != 0 && a.part) {
+          n_it += (uint32_t)work_item(plan, t).KB;
+        } else {
+          const int ks = t % a.KS;
+          n_it += (uint32_t)((int)((int64_t)KB_all * (ks + 1) / a.KS) - (int)((int64_t)KB_all * ks / a.KS));
+        }
       }
       for (uint32_t it = 0; it < n_it; ++it) {
         const uint32_t s = it % TC_STAGES, buf = it & 1;
@@ -344,6 +363,19 @@ moe_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
     uint32_t it = 0;
     bool ok = true;
     int ntile = 0;  // work items this CTA has finished
+    auto epi_bar = [&]() { asm volatile("bar.sync 1, %0;" ::"n"(TC_EPI_THREADS) : "memory"); };
+    auto epi_any = [&](bool p) {  // barrier of the epilogue warps: does p hold for any of their threads?
+      uint32_t any;
+      asm volatile(
+          "{\n\t.reg .pred p, r;\n\t"
+          "setp.ne.b32 p, %1, 0;\n\t"
+          "bar.red.or.pred r, 1, %2, p;\n\t"
+          "selp.u32 %0, 1, 0, r;\n\t}"
+          : "=r"(any)
+          : "r"((uint32_t)(p ? 1 : 0)), "n"(TC_EPI_THREADS)
+          : "memory");
+      return any != 0;
+    };
     for (int t = blockIdx.x; t < total_tiles; t += gridDim.x, ++ntile) {
       // the item (its integer divisions included), its expert and rows and the scales of its first two K blocks: left
       // in shared memory by the scout warp
@@ -469,6 +501,57 @@ moe_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
       } else {
         clear_acc();  // (a wait ran out: nothing below stores anything, but nothing reads an unset register either)
       }
+      if (MODE != 0 && t >= plan.whole) {
+        // A part of a shared tile (always this CTA's last item): the partial sums go to the CTA's slot (16 bytes per lane,
+        // consecutive over the warp; only rows that exist), the CTA counts itself in, and the one that comes last adds
+        // the parts up in K order - the order of the sum does not depend on who that is - and finishes the tile.  Nobody
+        // waits for another CTA.
+        if (epi_any(!ok)) {
+          ok = false;
+          break;
+        }
+        const int first = (t - plan.whole) / plan.parts * plan.parts;  // CTA of the tile's first part
+        float4* const slots = reinterpret_cast<float4*>(a.part) + (size_t)first * (a.part_slot / 4) +
+                              ((q * TC_CG + cg) * (TC_CW / 2) * 32 + lane);
+        if (valid) {
+          float4* p = slots + (size_t)(blockIdx.x - first) * (a.part_slot / 4);
+#pragma unroll
+          for (int i = 0; i < TC_CW / 2; ++i) {
+            const float2 p0 = unpack2(acc[i / (TC_CW / 4)][2 * (i % (TC_CW / 4))]), p1 = unpack2(acc[i / (TC_CW / 4)][2 * (i % (TC_CW / 4)) + 1]);
+            __stcg(p + i * 32, make_float4(p0.x, p0.y, p1.x, p1.y));
+          }
+        }
+        __threadfence();
+        epi_bar();
+        if (warp == 4 && lane == 0) {
+          int32_t* cnt = a.part_cnt + work_shared(plan, t);
+          const int last = atomicAdd(cnt, 1) == plan.parts - 1;
+          if (last) *cnt = 0;  // ready for the next launch
+          sh->part_last = last;
+          __threadfence();
+        }
+        epi_bar();
+        if (!sh->part_last) {
+          if (rows_out) {  // take the rows' destinations out of their slot all the same
+            if (!mbar_wait(smem_u32(&sh->dst_full), ntile & 1, abort_flag)) break;
+            __syncwarp();
+            if (lane == 0) mbar_arrive(smem_u32(&sh->dst_empty));
+          }
+          break;  // (the last item)
+        }
+        clear_acc();
+        for (int c = 0; c < plan.parts; ++c) {
+          const float4* p = slots + (size_t)c * (a.part_slot / 4);
+          if (valid) {
+#pragma unroll
+            for (int i = 0; i < TC_CW / 2; ++i) {
+              const float4 v = __ldcg(p + i * 32);
+              acc2_t &x = acc[i / (TC_CW / 4)][2 * (i % (TC_CW / 4))], &y = acc[i / (TC_CW / 4)][2 * (i % (TC_CW / 4)) + 1];
+              x.x += v.x, x.y += v.y, y.x += v.z, y.y += v.w;
+            }
+          }
+        }
+      }
       float amax = 0.f;
       if (MODE == 0) {
         // SiLU(gate) * up; the row's 128 values are split over TC_CG warps, which exchange their maxima through
@@ -484,20 +567,9 @@ moe_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
       }
       // One decision for all epilogue warps before anything that couples them (the named barriers of the tile end): a
       // warp whose wait ran out comes here like the others, and if any did, all of them leave together.
-      {
-        uint32_t any_bad;
-        asm volatile(
-            "{\n\t.reg .pred p, r;\n\t"
-            "setp.ne.b32 p, %1, 0;\n\t"
-            "bar.red.or.pred r, 1, %2, p;\n\t"
-            "selp.u32 %0, 1, 0, r;\n\t}"
-            : "=r"(any_bad)
-            : "r"((uint32_t)(ok ? 0 : 1)), "n"(TC_EPI_THREADS)
-            : "memory");
-        if (any_bad) {
-          ok = false;
-          break;
-        }
+      if (epi_any(!ok)) {
+        ok = false;
+        break;
       }
       // Results leave through shared memory.  A thread owns one row, so stores from registers would put 16 bytes per
       // lane into 32 different rows per instruction: half-used sectors (and, to a peer, 32 small packets), which cost
@@ -736,9 +808,18 @@ int launch_tc(const MoeGemmArgs& g, cudaStream_t st) {
     cudaFuncSetAttribute(moe_gemm_tc_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TC_SMEM_BYTES);
     di->attr_set = true;
   }
+  if (MODE != 0 && a.KS == 1 && !a.comb32 && !g.row_src && g.split.part) {
+    const int64_t rows = g.P / (g.E < g.P ? g.E : g.P);  // of an average tile
+    a.part = g.split.part;
+    a.part_cnt = g.split.cnt;
+    a.part_slot = moe_split_slot_floats(g.P);
+    a.part_rows = (int)(rows < kTileM ? rows : kTileM);
+  }
   const long long max_tiles = (long long)g.max_mtiles * a.NT * a.KS;
   const int sms = g.max_ctas > 0 && g.max_ctas < device_sm_count() ? g.max_ctas : device_sm_count();
-  const int grid = (int)(max_tiles < sms ? max_tiles : sms);
+  // (parts of shared tiles are items too)
+  const int grid = (int)((a.part ? max_tiles * kMaxParts : max_tiles) < sms ? (a.part ? max_tiles * kMaxParts : max_tiles) : sms);
+  if (grid > kMaxSplitCtas) a.part = nullptr;  // the slots are laid out for that many
   moe_gemm_tc_kernel<MODE><<<grid, TC_THREADS, TC_SMEM_BYTES, st>>>(tmA, tmB0, tmB1, a);
   return moe_launch_status();
 }

@@ -4,6 +4,18 @@
 
 constexpr int kTileM = 128;  // rows of one m-tile of the grouped GEMMs
 
+// Workspace of tiles that several CTAs share (schedule.h): partial sums, one slot per CTA, and one counter per shared
+// tile, zero when the launch starts and zero again when it ends.
+constexpr int kMaxSplitCtas = 160;
+constexpr int kSplitCounters = kMaxSplitCtas;
+struct MoeSplitBuffers {
+  float* part;
+  int32_t* cnt;
+};
+// floats of one slot: the row quarters of a 128 x 256 tile that a problem of P rows can have
+inline int moe_split_slot_floats(int64_t P) { return (int)(P < kTileM ? (P + 31) / 32 : kTileM / 32) * 32 * 256; }
+inline size_t moe_split_part_bytes(int64_t P) { return (size_t)kMaxSplitCtas * moe_split_slot_floats(P) * sizeof(float); }
+
 // One grouped-GEMM problem: rows [0,P) sorted by expert, m-tiles built from expert_offsets.
 struct MoeGemmArgs {
   // activations
@@ -35,6 +47,7 @@ struct MoeGemmArgs {
   __nv_bfloat16* out;       // gemm2: bf16 rows of H, row index = row_map ? row_map[r] : r
   int ksplit;               // gemm2 (tensor-core path): > 1 splits K over CTAs, partial sums added into out32
   float* out32;             // fp32 [rows,H], zero on entry, same row indexing as out (needed when ksplit > 1)
+  MoeSplitBuffers split;    // lets CTAs share tiles (part NULL = they may not)
   // gemm2 with the weighted combine fused in (tensor-core path only): row r adds comb_w[pair] * y[r,:] into
   // comb32[pair / div, :], pair = row_map ? row_map[r] : r; comb32 fp32 [T,H], zero on entry; comb_w NULL = weight 1
   float* comb32;
@@ -52,8 +65,13 @@ struct MoeIdentityLists {
   int32_t* offsets;
   int32_t* mtiles;
   int32_t* num_mtiles;
+  int32_t* split_cnt;  // kSplitCounters counters to clear, or NULL
 };
 #ifdef __CUDACC__
+__device__ __forceinline__ void moe_clear_counters(int32_t* cnt) {
+  if (cnt)
+    for (int i = threadIdx.x; i < kSplitCounters; i += blockDim.x) cnt[i] = 0;
+}
 // by the threads of one block
 __device__ __forceinline__ void moe_write_identity_lists(const MoeIdentityLists& l, int rows) {
   const int n = (rows + kTileM - 1) / kTileM;
@@ -61,6 +79,7 @@ __device__ __forceinline__ void moe_write_identity_lists(const MoeIdentityLists&
     l.mtiles[2 * i] = 0;
     l.mtiles[2 * i + 1] = i * kTileM;
   }
+  moe_clear_counters(l.split_cnt);
   if (threadIdx.x == 0) l.offsets[0] = 0, l.offsets[1] = rows, *l.num_mtiles = n;
 }
 #endif
@@ -68,15 +87,16 @@ __device__ __forceinline__ void moe_write_identity_lists(const MoeIdentityLists&
 // b200moe_permute that also writes the inverse map (pos_of, may be NULL) and the m-tile list when one CTA does the whole sort (at most 1024 pairs)
 int moe_permute_impl(int32_t* sorted_pair, int32_t* expert_offsets, const int32_t* ids, int64_t T, int64_t k, int64_t E,
                      int32_t* scratch, int32_t* status, int32_t* pos_of, int32_t* mtiles, int32_t* num_mtiles,
-                     int max_mtiles, bool* tiles_done, void* stream);
+                     int max_mtiles, int32_t* split_cnt, bool* tiles_done, void* stream);
 // quantised rows of x at the positions of every token's k pairs; quantised rows 0..rows with the identity lists
 int moe_quant_tokens(uint8_t* q, float* s_t, int64_t ld, const void* x, const int32_t* pos_of, int64_t T, int64_t k,
                      int64_t H, cudaStream_t st);
 int moe_quant_identity(uint8_t* q, float* s_t, int64_t ld, const void* x, int64_t rows, int64_t H,
                        const MoeIdentityLists& lists, cudaStream_t st);
-// tiles of rows [offsets[e], offsets[e+1]) clipped to max_rows; at most max_mtiles entries are written
+// tiles of rows [offsets[e], offsets[e+1]) clipped to max_rows; at most max_mtiles entries are written; clears the
+// counters of shared tiles (split_cnt, may be NULL)
 int moe_build_mtiles(int32_t* mtiles, int32_t* num_mtiles, const int32_t* offsets, int E, int64_t max_rows,
-                     int max_mtiles, cudaStream_t st);
+                     int max_mtiles, int32_t* split_cnt, cudaStream_t st);
 int moe_identity_lists(const MoeIdentityLists& lists, int64_t rows, cudaStream_t st);
 
 int moe_gemm1_simple(const MoeGemmArgs& a, int act_mode, cudaStream_t st);

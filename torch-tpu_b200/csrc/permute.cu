@@ -121,7 +121,8 @@ permute_scatter_kernel(const int32_t* __restrict__ ids, int64_t P, int E,
 __global__ void __launch_bounds__(kChunk)
 permute_small_kernel(const int32_t* __restrict__ ids, int64_t P, int E, int32_t* __restrict__ offsets,
                      int32_t* __restrict__ sorted_pair, int32_t* status, int32_t* __restrict__ mtiles,
-                     int32_t* __restrict__ num_mtiles, int max_mtiles, int32_t* __restrict__ pos_of) {
+                     int32_t* __restrict__ num_mtiles, int max_mtiles, int32_t* __restrict__ pos_of,
+                     int32_t* split_cnt) {
   extern __shared__ int wh[];
   __shared__ int tmp[kChunk];
   __shared__ int soffs[kMaxE + 1];
@@ -149,6 +150,7 @@ permute_small_kernel(const int32_t* __restrict__ ids, int64_t P, int E, int32_t*
   if (mtiles) {
     // the m-tile list of the grouped GEMMs ({expert, first row} per 128 rows of an expert) from the same offsets:
     // one launch less on the decode path
+    moe_clear_counters(split_cnt);
     __syncthreads();
     const int t = threadIdx.x;
     const int b = t < E ? soffs[t] : 0;
@@ -312,7 +314,7 @@ extern "C" size_t b200moe_permute_scratch_ints(int64_t P, int64_t E) {
 // *tiles_done is set (else the caller builds the list from expert_offsets)
 int moe_permute_impl(int32_t* sorted_pair, int32_t* expert_offsets, const int32_t* ids, int64_t T, int64_t k, int64_t E,
                      int32_t* scratch, int32_t* status, int32_t* pos_of, int32_t* mtiles, int32_t* num_mtiles,
-                     int max_mtiles, bool* tiles_done, void* stream) {
+                     int max_mtiles, int32_t* split_cnt, bool* tiles_done, void* stream) {
   if (tiles_done) *tiles_done = false;
   MOE_CHECK_ARG(sorted_pair && expert_offsets && ids && T >= 0 && k > 0 && E > 0);
   const int64_t P = T * k;
@@ -331,7 +333,7 @@ int moe_permute_impl(int32_t* sorted_pair, int32_t* expert_offsets, const int32_
   }
   if (P <= kChunk) {
     permute_small_kernel<<<1, kChunk, smem, st>>>(ids, P, (int)E, expert_offsets, sorted_pair, status, mtiles,
-                                                  num_mtiles, max_mtiles, pos_of);
+                                                  num_mtiles, max_mtiles, pos_of, split_cnt);
     if (tiles_done) *tiles_done = mtiles != nullptr;
     return moe_launch_status();
   }
@@ -347,7 +349,7 @@ int moe_permute_impl(int32_t* sorted_pair, int32_t* expert_offsets, const int32_
 extern "C" int b200moe_permute(int32_t* sorted_pair, int32_t* expert_offsets, const int32_t* ids, int64_t T,
                                int64_t k, int64_t E, int32_t* scratch, int32_t* status, void* stream) {
   return moe_permute_impl(sorted_pair, expert_offsets, ids, T, k, E, scratch, status, nullptr, nullptr, nullptr, 0,
-                          nullptr, stream);
+                          nullptr, nullptr, stream);
 }
 
 extern "C" int b200moe_gather_scatter_index(int32_t* gather_index, int32_t* scatter_index,
