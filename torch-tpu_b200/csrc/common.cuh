@@ -33,6 +33,50 @@ static inline int moe_launch_status() {
 
 static inline bool moe_aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
+// ---- launches that overlap the end of the kernel before them -----------------------------------------------------
+// A call is a chain of short kernels, and at decode sizes the gaps between them (drain, launch, set-up of the next) cost
+// as much as the kernels.  moe_launch starts a kernel while its predecessor on the stream still runs (programmatic stream
+// serialisation).  The rules that make this safe: every kernel launched this way executes pdl_wait() in every thread
+// before it touches memory that an earlier kernel of the stream writes or reads (it returns when the predecessor has
+// completed and its writes are visible), and pdl_next(), which lets the successor start, comes after it.  So when a
+// kernel starts, everything before its direct predecessor is complete.  Launched after anything else than such a
+// kernel, pdl_wait() finds its predecessor complete.
+#ifdef __CUDACC__
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_begin() {
+  pdl_wait();
+  pdl_next();
+}
+template <typename... KArgs, typename... Args>
+inline int moe_launch_cluster(int cluster_y, void (*kernel)(KArgs...), dim3 grid, unsigned block, size_t smem,
+                              cudaStream_t st, Args&&... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute at[2];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  at[1].id = cudaLaunchAttributeClusterDimension;
+  at[1].val.clusterDim.x = at[1].val.clusterDim.z = 1;
+  at[1].val.clusterDim.y = (unsigned)cluster_y;
+  cfg.attrs = at;
+  cfg.numAttrs = cluster_y > 1 ? 2 : 1;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    return (int)e;
+  }
+  return B200MOE_OK;
+}
+template <typename... KArgs, typename... Args>
+inline int moe_launch(void (*kernel)(KArgs...), dim3 grid, unsigned block, size_t smem, cudaStream_t st, Args&&... args) {
+  return moe_launch_cluster(1, kernel, grid, block, smem, st, static_cast<Args&&>(args)...);
+}
+#endif
+
 // ---- scalar loads of score / scale tensors in their storage dtype -----------------------------
 __device__ __forceinline__ float moe_load_as_f32(const void* p, int64_t i, int dtype) {
   if (dtype == B200MOE_F32) return reinterpret_cast<const float*>(p)[i];

@@ -105,6 +105,7 @@ WsLayout make_layout(const b200moe_experts_desc& d) {
 
 __global__ void scales_to_f32_kernel(float* __restrict__ dst, const __nv_bfloat16* __restrict__ a,
                                      const __nv_bfloat16* __restrict__ b, const __nv_bfloat16* __restrict__ c, int64_t n) {
+  pdl_begin();
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) {
     dst[i] = __bfloat162float(a[i]);
@@ -217,12 +218,17 @@ extern "C" int b200moe_experts(void* out, const void* x, const void* w_gate, con
   // The fork is recorded before any routed work is queued, so both passes start together; they share no workspace
   // region.  One call per device at a time may use the side stream (calls on one device are expected to be queued
   // from one host thread).
-  // fused combine: the sums of the routed AND the shared expert meet in this buffer, so it is cleared before the
-  // side stream forks off
+  // The sums of the routed AND the shared expert meet in the fused combine's buffer: it is cleared before the side stream
+  // forks off.
   float* acc32 = reinterpret_cast<float*>(ws + L.acc32);
-  if (fused && do_g2) cudaMemsetAsync(acc32, 0, (size_t)d->T * d->H * sizeof(float), st);
   SideStream* side = (d->I_shared > 0 && use_tc && d->T <= kSharedOverlapMaxTokens && stages == B200MOE_STAGE_ALL)
                          ? side_stream() : nullptr;
+  // the fused combine's rows are cleared by the quantisation kernel, or here where that does not run or comes too late
+  const bool clear_in_quant = fused && w8a8 && do_prep && !side;
+  if (fused && do_g2 && !clear_in_quant) {
+    const cudaError_t e = cudaMemsetAsync(acc32, 0, (size_t)d->T * d->H * sizeof(float), st);
+    if (e != cudaSuccess) return (int)e;
+  }
   if (side) {
     if (cudaEventRecord(side->fork, st) != cudaSuccess || cudaStreamWaitEvent(side->s, side->fork, 0) != cudaSuccess)
       return (int)cudaGetLastError();
@@ -240,17 +246,16 @@ extern "C" int b200moe_experts(void* out, const void* x, const void* w_gate, con
   }
   if (w8a8 && do_prep) {
     rc = moe_quant_tokens(reinterpret_cast<uint8_t*>(ws + L.xq), reinterpret_cast<float*>(ws + L.xs), L.ld, x,
-                          I32(L.pos_of), d->T, d->k, d->H, st);
+                          I32(L.pos_of), d->T, d->k, d->H, clear_in_quant ? acc32 : nullptr, st);
     if (rc) return rc;
   }
 
   const bool cvt = d->scale_dtype == B200MOE_BF16 && (tc1 || tc2);
   const int64_t nsc = d->E * (d->I / kBlock) * (d->H / kBlock);
   if (cvt && do_prep) {
-    scales_to_f32_kernel<<<(unsigned)((nsc + 255) / 256), 256, 0, st>>>(
+    rc = moe_launch(scales_to_f32_kernel, (unsigned)((nsc + 255) / 256), 256, 0, st,
         reinterpret_cast<float*>(ws + L.sc32), reinterpret_cast<const __nv_bfloat16*>(s_gate),
         reinterpret_cast<const __nv_bfloat16*>(s_up), reinterpret_cast<const __nv_bfloat16*>(s_down), nsc);
-    rc = moe_launch_status();
     if (rc) return rc;
   }
   const float* sc32 = reinterpret_cast<const float*>(ws + L.sc32);
@@ -281,6 +286,7 @@ extern "C" int b200moe_experts(void* out, const void* x, const void* w_gate, con
   g.hs_t = reinterpret_cast<float*>(ws + L.hs);
   g.h16 = reinterpret_cast<__nv_bfloat16*>(ws + L.hq);
   if (w8a8) g.split = MoeSplitBuffers{reinterpret_cast<float*>(ws + L.part), I32(L.cnt)};
+  g.lists_ready = 1;  // the permutation's, with at least the quantisation kernel in between
   g.status = status;
   __nv_bfloat16* xg = reinterpret_cast<__nv_bfloat16*>(ws + L.xq);  // W8A16 tensor-core path: x rows in sorted order
   if (tc1_16 && do_prep) {
@@ -346,11 +352,10 @@ extern "C" int b200moe_experts(void* out, const void* x, const void* w_gate, con
     }
     const int64_t nscs = (d->I_shared / kBlock) * (d->H / kBlock);
     if (cvt && do_prep) {
-      scales_to_f32_kernel<<<(unsigned)((nscs + 255) / 256), 256, 0, ss>>>(
+      rc = moe_launch(scales_to_f32_kernel, (unsigned)((nscs + 255) / 256), 256, 0, ss,
           reinterpret_cast<float*>(ws + L.s_sc32), reinterpret_cast<const __nv_bfloat16*>(shared_s_gate),
           reinterpret_cast<const __nv_bfloat16*>(shared_s_up), reinterpret_cast<const __nv_bfloat16*>(shared_s_down),
           nscs);
-      rc = moe_launch_status();
       if (rc) return rc;
     }
     const float* ssc32 = reinterpret_cast<const float*>(ws + L.s_sc32);
@@ -372,6 +377,7 @@ extern "C" int b200moe_experts(void* out, const void* x, const void* w_gate, con
     s.P = d->T;
     s.I = (int)d->I_shared;
     s.E = 1;
+    s.lists_ready = 0;  // written by the quantisation kernel, which may be the direct predecessor
     if (w8a8) s.split = MoeSplitBuffers{reinterpret_cast<float*>(ws + L.s_part), I32(L.s_cnt)};
     s.hq = reinterpret_cast<uint8_t*>(ws + L.s_hq);
     s.hs_t = reinterpret_cast<float*>(ws + L.s_hs);
@@ -389,6 +395,7 @@ extern "C" int b200moe_experts(void* out, const void* x, const void* w_gate, con
     }
     if (rc) return rc;
     MoeGemmArgs s2 = s;
+    s2.lists_ready = do_g1;  // the gate/up GEMM is in between
     s2.aq = s.hq;
     s2.as_t = s.hs_t;
     s2.a16 = s.h16;
@@ -499,10 +506,9 @@ int grouped_mlp_impl(void* y, const uint8_t* xq, const float* xs_t, int64_t ld, 
   if (use_tc && scale_dtype == B200MOE_BF16) {
     const int64_t nsc = E * (I / kBlock) * (H / kBlock);
     float* sc32 = reinterpret_cast<float*>(ws + L.sc32);
-    scales_to_f32_kernel<<<(unsigned)((nsc + 255) / 256), 256, 0, st>>>(
+    rc = moe_launch(scales_to_f32_kernel, (unsigned)((nsc + 255) / 256), 256, 0, st,
         sc32, reinterpret_cast<const __nv_bfloat16*>(s_gate), reinterpret_cast<const __nv_bfloat16*>(s_up),
         reinterpret_cast<const __nv_bfloat16*>(s_down), nsc);
-    rc = moe_launch_status();
     if (rc) return rc;
     sg = sc32, su = sc32 + nsc, sd = sc32 + 2 * nsc, sdt = B200MOE_F32;
   }
@@ -531,6 +537,7 @@ int grouped_mlp_impl(void* y, const uint8_t* xq, const float* xs_t, int64_t ld, 
   rc = use_tc ? moe_gemm1_tc(g, st) : moe_gemm1_simple(g, B200MOE_ACT_W8A8, st);
   if (rc) return rc;
   MoeGemmArgs g2 = g;
+  g2.lists_ready = 1;  // the gate/up GEMM is in between
   g2.aq = g.hq;
   g2.as_t = g.hs_t;
   g2.row_map = row_map;
@@ -597,6 +604,7 @@ LinLayout lin_layout(int64_t M, int64_t K, int64_t N, int scale_dtype) {
   return L;
 }
 __global__ void scales1_to_f32_kernel(float* __restrict__ dst, const __nv_bfloat16* __restrict__ s, int64_t n) {
+  pdl_begin();
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) dst[i] = __bfloat162float(s[i]);
 }
@@ -632,9 +640,8 @@ extern "C" int b200moe_linear_w8(void* out, const void* x, const void* w, const 
   const void* sc = scale;
   if (scale_dtype == B200MOE_BF16) {
     const int64_t n = ((N + kBlock - 1) / kBlock) * (K / kBlock);
-    scales1_to_f32_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(
+    rc = moe_launch(scales1_to_f32_kernel, (unsigned)((n + 255) / 256), 256, 0, st,
         reinterpret_cast<float*>(ws + L.sc32), reinterpret_cast<const __nv_bfloat16*>(scale), n);
-    rc = moe_launch_status();
     if (rc) return rc;
     sc = ws + L.sc32;
   }
@@ -663,6 +670,7 @@ extern "C" int b200moe_linear_w8(void* out, const void* x, const void* w, const 
 // ---- FP8 x FP8 matrix product with one scale per operand ------------------------------------------------------------
 namespace {
 __global__ void fill_scalar_scale_kernel(float* __restrict__ dst, const float* __restrict__ scale, int64_t n) {
+  pdl_begin();
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) dst[i] = scale ? *scale : 1.0f;
 }
@@ -722,9 +730,11 @@ extern "C" int b200moe_scaled_mm(void* out, int out_dtype, const void* a, const 
   if (rc) return rc;
   // the kernel applies act_scale[row,kb] * weight_scale[nb,kb] to every 128-deep partial sum: constant grids here
   const int64_t nxs = (K / kBlock) * L.ld, nws = ((N + kBlock - 1) / kBlock) * (K / kBlock);
-  fill_scalar_scale_kernel<<<(unsigned)((nxs + 255) / 256), 256, 0, st>>>(reinterpret_cast<float*>(ws + L.xs), scale_a, nxs);
-  fill_scalar_scale_kernel<<<(unsigned)((nws + 255) / 256), 256, 0, st>>>(reinterpret_cast<float*>(ws + L.ws), scale_b, nws);
-  rc = moe_launch_status();
+  rc = moe_launch(fill_scalar_scale_kernel, (unsigned)((nxs + 255) / 256), 256, 0, st, reinterpret_cast<float*>(ws + L.xs),
+                  scale_a, nxs);
+  if (rc) return rc;
+  rc = moe_launch(fill_scalar_scale_kernel, (unsigned)((nws + 255) / 256), 256, 0, st, reinterpret_cast<float*>(ws + L.ws),
+                  scale_b, nws);
   if (rc) return rc;
   MoeGemmArgs g{};
   g.aq = reinterpret_cast<const uint8_t*>(a);

@@ -130,6 +130,7 @@ moe_gemm_bf16_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_co
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = sh->tmem_base;
+  pdl_begin();
 
   const int num_mtiles = *a.num_mtiles;
   const int total_tiles = num_mtiles * a.NT;
@@ -481,14 +482,14 @@ int launch_bt(const MoeGemmArgs& g, cudaStream_t st) {
   const long long max_tiles = (long long)g.max_mtiles * a.NT;
   const int sms = g.max_ctas > 0 && g.max_ctas < moe_device_sm_count() ? g.max_ctas : moe_device_sm_count();
   const int grid = (int)(max_tiles < sms ? max_tiles : sms);
-  moe_gemm_bf16_tc_kernel<GEMM2><<<grid, BT_THREADS, BT_SMEM_BYTES, st>>>(tmA, tmB0, tmB1, a);
-  return moe_launch_status();
+  return moe_launch(moe_gemm_bf16_tc_kernel<GEMM2>, grid, BT_THREADS, BT_SMEM_BYTES, st, tmA, tmB0, tmB1, a);
 }
 
 // gather of bf16 rows into sorted order: dst[r,:] = x[row_map[r] / div, :] (16-byte accesses; one warp per row)
 __global__ void __launch_bounds__(256)
 gather_rows_bf16_kernel(__nv_bfloat16* __restrict__ dst, const __nv_bfloat16* __restrict__ x,
                         const int32_t* __restrict__ row_map, int div, int64_t rows, int H) {
+  pdl_begin();
   const int lane = threadIdx.x & 31;
   const int64_t r = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
   if (r >= rows) return;
@@ -504,8 +505,7 @@ gather_rows_bf16_kernel(__nv_bfloat16* __restrict__ dst, const __nv_bfloat16* __
 int moe_gather_rows_bf16(__nv_bfloat16* dst, const __nv_bfloat16* x, const int32_t* row_map, int div, int64_t rows,
                          int H, cudaStream_t st) {
   if (rows == 0) return B200MOE_OK;
-  gather_rows_bf16_kernel<<<(unsigned)((rows + 7) / 8), 256, 0, st>>>(dst, x, row_map, div, rows, H);
-  return moe_launch_status();
+  return moe_launch(gather_rows_bf16_kernel, (unsigned)((rows + 7) / 8), 256, 0, st, dst, x, row_map, div, rows, H);
 }
 int moe_gemm1_w8a16_tc(const MoeGemmArgs& a, cudaStream_t st) { return launch_bt<false>(a, st); }
 int moe_gemm2_w8a16_tc(const MoeGemmArgs& a, cudaStream_t st) { return launch_bt<true>(a, st); }

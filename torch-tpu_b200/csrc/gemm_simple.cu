@@ -14,6 +14,7 @@ __device__ __forceinline__ float scale_at(const void* s, int64_t i, int dtype) {
 
 template <int ACT>
 __global__ void __launch_bounds__(256) gemm1_simple_kernel(MoeGemmArgs a) {
+  pdl_begin();
   __shared__ float sA[SR][SKC + 1];
   __shared__ float sG[128][SKC + 1];
   __shared__ float sU[128][SKC + 1];
@@ -131,6 +132,7 @@ __global__ void __launch_bounds__(256) gemm1_simple_kernel(MoeGemmArgs a) {
 
 template <int ACT>
 __global__ void __launch_bounds__(256) gemm2_simple_kernel(MoeGemmArgs a) {
+  pdl_begin();
   __shared__ float sA[SR][SKC + 1];
   __shared__ float sB[SKC][128];
   const int nt = blockIdx.x;
@@ -201,6 +203,7 @@ __global__ void __launch_bounds__(256) gemm2_simple_kernel(MoeGemmArgs a) {
 __global__ void __launch_bounds__(1024)
 build_mtiles_kernel(int32_t* __restrict__ mtiles, int32_t* __restrict__ num_mtiles,
                     const int32_t* __restrict__ offsets, int E, int max_rows, int max_mtiles, int32_t* split_cnt) {
+  pdl_begin();
   moe_clear_counters(split_cnt);
   __shared__ int tmp[1024];
   const int t = threadIdx.x;
@@ -228,6 +231,7 @@ build_mtiles_kernel(int32_t* __restrict__ mtiles, int32_t* __restrict__ num_mtil
 }
 
 __global__ void __launch_bounds__(256) identity_lists_kernel(MoeIdentityLists lists, int rows) {
+  pdl_begin();
   moe_write_identity_lists(lists, rows);
 }
 
@@ -239,6 +243,7 @@ __global__ void __launch_bounds__(256)
 combine_kernel(__nv_bfloat16* __restrict__ out, const __nv_bfloat16* __restrict__ y, const void* __restrict__ w,
                int w_dtype, const __nv_bfloat16* __restrict__ add, const int32_t* __restrict__ pos,
                const int32_t* __restrict__ ids, int E, int64_t T, int k, int H) {
+  pdl_begin();
   const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int hv = H / 8;
   if (idx >= T * hv) return;
@@ -297,27 +302,23 @@ combine_kernel(__nv_bfloat16* __restrict__ out, const __nv_bfloat16* __restrict_
 
 int moe_build_mtiles(int32_t* mtiles, int32_t* num_mtiles, const int32_t* offsets, int E, int64_t max_rows,
                      int max_mtiles, int32_t* split_cnt, cudaStream_t st) {
-  build_mtiles_kernel<<<1, 1024, 0, st>>>(mtiles, num_mtiles, offsets, E, (int)max_rows, max_mtiles, split_cnt);
-  return moe_launch_status();
+  return moe_launch(build_mtiles_kernel, 1, 1024, 0, st, mtiles, num_mtiles, offsets, E, (int)max_rows, max_mtiles, split_cnt);
 }
 
 int moe_identity_lists(const MoeIdentityLists& lists, int64_t rows, cudaStream_t st) {
-  identity_lists_kernel<<<1, 256, 0, st>>>(lists, (int)rows);
-  return moe_launch_status();
+  return moe_launch(identity_lists_kernel, 1, 256, 0, st, lists, (int)rows);
 }
 
 int moe_gemm1_simple(const MoeGemmArgs& a, int act_mode, cudaStream_t st) {
   dim3 grid((unsigned)(a.I / 128), (unsigned)(a.max_mtiles * 8));
-  if (act_mode == B200MOE_ACT_W8A8) gemm1_simple_kernel<B200MOE_ACT_W8A8><<<grid, 256, 0, st>>>(a);
-  else gemm1_simple_kernel<B200MOE_ACT_W8A16><<<grid, 256, 0, st>>>(a);
-  return moe_launch_status();
+  return moe_launch(act_mode == B200MOE_ACT_W8A8 ? gemm1_simple_kernel<B200MOE_ACT_W8A8> : gemm1_simple_kernel<B200MOE_ACT_W8A16>,
+                    grid, 256, 0, st, a);
 }
 
 int moe_gemm2_simple(const MoeGemmArgs& a, int act_mode, cudaStream_t st) {
   dim3 grid((unsigned)(a.H / 128), (unsigned)(a.max_mtiles * 8));
-  if (act_mode == B200MOE_ACT_W8A8) gemm2_simple_kernel<B200MOE_ACT_W8A8><<<grid, 256, 0, st>>>(a);
-  else gemm2_simple_kernel<B200MOE_ACT_W8A16><<<grid, 256, 0, st>>>(a);
-  return moe_launch_status();
+  return moe_launch(act_mode == B200MOE_ACT_W8A8 ? gemm2_simple_kernel<B200MOE_ACT_W8A8> : gemm2_simple_kernel<B200MOE_ACT_W8A16>,
+                    grid, 256, 0, st, a);
 }
 
 extern "C" int b200moe_combine_masked(void* out, const void* y, const int32_t* pos, const void* w, int w_dtype,
@@ -329,10 +330,9 @@ extern "C" int b200moe_combine_masked(void* out, const void* y, const int32_t* p
   if (!moe_aligned16(out) || !moe_aligned16(y) || (add && !moe_aligned16(add))) return B200MOE_EALIGN;
   if (T == 0) return B200MOE_OK;
   const int64_t n = T * (H / 8);
-  combine_kernel<<<(unsigned)((n + 255) / 256), 256, 0, (cudaStream_t)stream>>>(
-      reinterpret_cast<__nv_bfloat16*>(out), reinterpret_cast<const __nv_bfloat16*>(y), w, w_dtype,
-      reinterpret_cast<const __nv_bfloat16*>(add), pos, ids, (int)E, T, (int)k, (int)H);
-  return moe_launch_status();
+  return moe_launch(combine_kernel, (unsigned)((n + 255) / 256), 256, 0, (cudaStream_t)stream,
+                    reinterpret_cast<__nv_bfloat16*>(out), reinterpret_cast<const __nv_bfloat16*>(y), w, w_dtype,
+                    reinterpret_cast<const __nv_bfloat16*>(add), pos, ids, (int)E, T, (int)k, (int)H);
 }
 
 extern "C" int b200moe_combine_indexed(void* out, const void* y, const int32_t* pos, const void* w, int w_dtype,

@@ -95,6 +95,7 @@ struct TcArgs {
   float* part;
   int32_t* part_cnt;
   int part_slot, part_rows;
+  int lists_ready;  // mtiles, num_mtiles and offsets may be read before pdl_wait()
   int m_major;   // work-item order: 0 = n-tile slow, m-tile fast; 1 = m-tile slow, n-tile fast (see launch_tc)
   float* out32;  // fp32 accumulation target when KS > 1; with KS == 1 (linear layer only): fp32 rows stored instead of bf16
   // down GEMM with the weighted combine fused in: row r adds comb_w[pair] * y[r,:] into comb32[pair / div, :] (fp32,
@@ -173,6 +174,9 @@ moe_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = sh->tmem_base;
+  // Everything above overlaps the end of the kernel before this one.  Where the work list is older than that kernel, the
+  // producer also requests its first weight tiles before the wait (they are nobody's output).
+  if (!a.lists_ready) pdl_wait();
 
   const int num_mtiles = *a.num_mtiles;
   const int KB_all = (GEMM2 ? a.I : a.H) / kBlock;
@@ -229,6 +233,31 @@ moe_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
         nx = item_of(blockIdx.x);
         nx_e = a.mtiles[2 * nx.mt], nx_row0 = a.mtiles[2 * nx.mt + 1];
       }
+      auto load_b = [&](int nt, int e, int kb, uint32_t sb, uint32_t full) {
+        if (DENSE) {
+          tma_load_2d(sb, &tmB0, kb * kBlock, e * a.I + nt * 256, full);
+          tma_load_2d(sb + 128 * 128, &tmB0, kb * kBlock, e * a.I + nt * 256 + 128, full);
+        } else if (!GEMM2) {
+          tma_load_2d(sb, &tmB0, kb * kBlock, e * a.I + nt * 128, full);
+          tma_load_2d(sb + 128 * 128, &tmB1, kb * kBlock, e * a.I + nt * 128, full);
+        } else {
+          tma_load_2d(sb, &tmB0, nt * 256, e * a.I + kb * kBlock, full);
+          tma_load_2d(sb + 128 * 128, &tmB0, nt * 256 + 128, e * a.I + kb * kBlock, full);
+        }
+      };
+      // the first item's first weight tiles; their A tiles follow after the wait (the ring is empty: no stage to wait for)
+      uint32_t n_early = 0;
+      if (a.lists_ready) {
+        if ((int)blockIdx.x < total_tiles) {
+          n_early = nx.KB < TC_STAGES ? nx.KB : TC_STAGES;
+          for (uint32_t s = 0; s < n_early; ++s) {
+            const uint32_t full = smem_u32(&sh->full[s]);
+            mbar_arrive_expect_tx(full, TC_STAGE_BYTES);
+            load_b(nx.nt, nx_e, nx.kb0 + s, smem_base + s * TC_STAGE_BYTES + TC_A_BYTES, full);
+          }
+        }
+        pdl_wait();
+      }
       for (int t = blockIdx.x; t < total_tiles && ok; t += gridDim.x) {
         const int nt = nx.nt, kb0 = nx.kb0, kb1 = nx.kb0 + nx.KB;
         const int e = nx_e, row0 = nx_row0;
@@ -239,24 +268,19 @@ moe_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
         for (int kb = kb0; kb < kb1; ++kb, ++it) {
           const int s = it % TC_STAGES;
           const uint32_t ph = (it / TC_STAGES) & 1;
+          const uint32_t full = smem_u32(&sh->full[s]);
+          const uint32_t sa = smem_base + s * TC_STAGE_BYTES, sb = sa + TC_A_BYTES;
+          if (it < n_early) {
+            tma_load_2d(sa, &tmA, kb * kBlock, row0, full);
+            continue;
+          }
           if (!mbar_wait(smem_u32(&sh->empty[s]), ph ^ 1, abort_flag)) {
             ok = false;
             break;
           }
-          const uint32_t full = smem_u32(&sh->full[s]);
-          const uint32_t sa = smem_base + s * TC_STAGE_BYTES, sb = sa + TC_A_BYTES;
           mbar_arrive_expect_tx(full, TC_STAGE_BYTES);
           tma_load_2d(sa, &tmA, kb * kBlock, row0, full);
-          if (DENSE) {
-            tma_load_2d(sb, &tmB0, kb * kBlock, e * a.I + nt * 256, full);
-            tma_load_2d(sb + 128 * 128, &tmB0, kb * kBlock, e * a.I + nt * 256 + 128, full);
-          } else if (!GEMM2) {
-            tma_load_2d(sb, &tmB0, kb * kBlock, e * a.I + nt * 128, full);
-            tma_load_2d(sb + 128 * 128, &tmB1, kb * kBlock, e * a.I + nt * 128, full);
-          } else {
-            tma_load_2d(sb, &tmB0, nt * 256, e * a.I + kb * kBlock, full);
-            tma_load_2d(sb + 128 * 128, &tmB0, nt * 256 + 128, e * a.I + kb * kBlock, full);
-          }
+          load_b(nt, e, kb, sb, full);
         }
       }
     }
@@ -303,6 +327,7 @@ moe_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
     // the scales of the first two K blocks): 2000 to 3000 cycles when an epilogue warp walks them at the start of the
     // item, a tenth of a short item, and the epilogue's K loop has no registers to carry them ahead.  This warp walks
     // them one item ahead and leaves them in shared memory.
+    pdl_wait();
     bool ok = true;
     uint32_t n = 0;
     for (int t = blockIdx.x; t < total_tiles && ok; t += gridDim.x, ++n) {
@@ -355,7 +380,10 @@ moe_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
         if (lane == 0) mbar_arrive(smem_u32(&sh->dst_full));
       }
     }
+  } else if (warp == 3) {
+    pdl_begin();  // let the next kernel's CTAs come up as this one's leave
   } else if (warp >= 4) {
+    pdl_wait();
     // ------------------------------------------------------------------ epilogue (4 * TC_CG warps)
     asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(TC_REG_HI));
     const int q = warp & 3, cg = (warp - 4) >> 2;
@@ -820,8 +848,8 @@ int launch_tc(const MoeGemmArgs& g, cudaStream_t st) {
   // (parts of shared tiles are items too)
   const int grid = (int)((a.part ? max_tiles * kMaxParts : max_tiles) < sms ? (a.part ? max_tiles * kMaxParts : max_tiles) : sms);
   if (grid > kMaxSplitCtas) a.part = nullptr;  // the slots are laid out for that many
-  moe_gemm_tc_kernel<MODE><<<grid, TC_THREADS, TC_SMEM_BYTES, st>>>(tmA, tmB0, tmB1, a);
-  return moe_launch_status();
+  a.lists_ready = g.lists_ready;
+  return moe_launch(moe_gemm_tc_kernel<MODE>, grid, TC_THREADS, TC_SMEM_BYTES, st, tmA, tmB0, tmB1, a);
 }
 
 }  // namespace
@@ -833,6 +861,7 @@ bool moe_tc_available() {
 
 namespace {
 __global__ void f32_rows_to_bf16_kernel(__nv_bfloat16* __restrict__ out, const float* __restrict__ in, int64_t n) {
+  pdl_begin();
   const int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * 4;
   if (i + 3 < n) {
     const float4 v = *reinterpret_cast<const float4*>(in + i);
@@ -843,8 +872,7 @@ __global__ void f32_rows_to_bf16_kernel(__nv_bfloat16* __restrict__ out, const f
 }  // namespace
 
 int moe_f32_rows_to_bf16(__nv_bfloat16* out, const float* in, int64_t n, cudaStream_t st) {
-  f32_rows_to_bf16_kernel<<<(unsigned)((n / 4 + 255) / 256), 256, 0, st>>>(out, in, n);
-  return moe_launch_status();
+  return moe_launch(f32_rows_to_bf16_kernel, (unsigned)((n / 4 + 255) / 256), 256, 0, st, out, in, n);
 }
 
 int moe_device_sm_count() { return device_sm_count(); }

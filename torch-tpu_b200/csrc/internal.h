@@ -57,6 +57,7 @@ struct MoeGemmArgs {
   // of that rank's buffer out_tbl[rank] (bf16 rows of H); overrides out/row_map
   const int32_t* row_src;
   const uint64_t* out_tbl;
+  int lists_ready;          // mtiles / num_mtiles / offsets are older than the launch's direct predecessor (see pdl_wait)
   int32_t* status;
 };
 
@@ -88,9 +89,9 @@ __device__ __forceinline__ void moe_write_identity_lists(const MoeIdentityLists&
 int moe_permute_impl(int32_t* sorted_pair, int32_t* expert_offsets, const int32_t* ids, int64_t T, int64_t k, int64_t E,
                      int32_t* scratch, int32_t* status, int32_t* pos_of, int32_t* mtiles, int32_t* num_mtiles,
                      int max_mtiles, int32_t* split_cnt, bool* tiles_done, void* stream);
-// quantised rows of x at the positions of every token's k pairs; quantised rows 0..rows with the identity lists
+// quantised rows of x at the positions of every token's k pairs (and zeros to acc32 [T,H], may be NULL); quantised rows 0..rows with the identity lists
 int moe_quant_tokens(uint8_t* q, float* s_t, int64_t ld, const void* x, const int32_t* pos_of, int64_t T, int64_t k,
-                     int64_t H, cudaStream_t st);
+                     int64_t H, float* acc32, cudaStream_t st);
 int moe_quant_identity(uint8_t* q, float* s_t, int64_t ld, const void* x, int64_t rows, int64_t H,
                        const MoeIdentityLists& lists, cudaStream_t st);
 // tiles of rows [offsets[e], offsets[e+1]) clipped to max_rows; at most max_mtiles entries are written; clears the

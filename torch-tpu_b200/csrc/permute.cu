@@ -41,6 +41,7 @@ __device__ __forceinline__ int chunk_hist(const int32_t* __restrict__ ids, int64
 __global__ void __launch_bounds__(kChunk)
 permute_hist_kernel(const int32_t* __restrict__ ids, int64_t P, int E, int32_t* __restrict__ chunk_cnt,
                     int32_t* status) {
+  pdl_begin();
   extern __shared__ int wh[];
   int rank;
   chunk_hist(ids, P, E, (int64_t)blockIdx.x * kChunk + threadIdx.x, wh, rank, status);
@@ -69,6 +70,7 @@ __device__ __forceinline__ void block_exclusive_scan(int my, int E, int32_t* __r
 
 __global__ void __launch_bounds__(kChunk)
 permute_scan_kernel(int32_t* __restrict__ chunk_cnt, int nchunks, int E, int32_t* __restrict__ offsets) {
+  pdl_begin();
   __shared__ int tmp[kChunk];
   int total = 0;
   if ((int)threadIdx.x < E) {
@@ -92,6 +94,7 @@ __global__ void __launch_bounds__(kChunk)
 permute_scatter_kernel(const int32_t* __restrict__ ids, int64_t P, int E,
                        const int32_t* __restrict__ chunk_base, const int32_t* __restrict__ offsets,
                        int32_t* __restrict__ sorted_pair, int32_t* __restrict__ pos_of) {
+  pdl_begin();
   extern __shared__ int wh[];
   int rank;
   const int64_t p = (int64_t)blockIdx.x * kChunk + threadIdx.x;
@@ -123,6 +126,7 @@ permute_small_kernel(const int32_t* __restrict__ ids, int64_t P, int E, int32_t*
                      int32_t* __restrict__ sorted_pair, int32_t* status, int32_t* __restrict__ mtiles,
                      int32_t* __restrict__ num_mtiles, int max_mtiles, int32_t* __restrict__ pos_of,
                      int32_t* split_cnt) {
+  pdl_begin();
   extern __shared__ int wh[];
   __shared__ int tmp[kChunk];
   __shared__ int soffs[kMaxE + 1];
@@ -171,6 +175,7 @@ __global__ void gather_scatter_index_kernel(int32_t* __restrict__ gather_index,
                                             int32_t* __restrict__ num_per_expert,
                                             const int32_t* __restrict__ sorted_pair,
                                             const int32_t* __restrict__ offsets, int64_t T, int k) {
+  pdl_begin();
   const int e = blockIdx.x;
   const int b = offsets[e], n = offsets[e + 1] - b;
   if (threadIdx.x == 0) num_per_expert[e] = n;
@@ -190,6 +195,7 @@ __global__ void __launch_bounds__(256)
 quant_rows_kernel(uint8_t* __restrict__ q, float* __restrict__ s_t, int64_t ld,
                   const __nv_bfloat16* __restrict__ x, const int32_t* __restrict__ row_map, int div,
                   int64_t rows, int H, int cpw, int warps_per_row, MoeIdentityLists lists) {
+  pdl_begin();
   if (lists.offsets && blockIdx.x == 0) moe_write_identity_lists(lists, (int)rows);
   const int lane = threadIdx.x & 31;
   const int64_t w = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
@@ -247,7 +253,9 @@ quant_rows_kernel(uint8_t* __restrict__ q, float* __restrict__ s_t, int64_t ld,
 constexpr int QT_CPW = 2;
 __global__ void __launch_bounds__(256)
 quant_tokens_kernel(uint8_t* __restrict__ q, float* __restrict__ s_t, int64_t ld, const __nv_bfloat16* __restrict__ x,
-                    const int32_t* __restrict__ pos_of, int64_t T, int k, int H, int cpw, int warps_per_tok) {
+                    const int32_t* __restrict__ pos_of, int64_t T, int k, int H, int cpw, int warps_per_tok,
+                    float* __restrict__ acc32) {
+  pdl_begin();
   const int lane = threadIdx.x & 31;
   const int64_t w = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
   const int64_t t = w / warps_per_tok;
@@ -260,6 +268,13 @@ quant_tokens_kernel(uint8_t* __restrict__ q, float* __restrict__ s_t, int64_t ld
     const bool on = u < cpw && c < H;
     raw[u][0] = on ? *reinterpret_cast<const uint4*>(x + t * H + c) : make_uint4(0, 0, 0, 0);
     raw[u][1] = on ? *reinterpret_cast<const uint4*>(x + t * H + c + 8) : make_uint4(0, 0, 0, 0);
+  }
+  if (acc32) {  // the token's fp32 row of the fused combine starts from zero
+#pragma unroll
+    for (int u = 0; u < QT_CPW; ++u)
+      if (u < cpw && c0 + u * 512 < H)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) reinterpret_cast<float4*>(acc32 + t * H + c0 + u * 512)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
   }
   int32_t my_pos = lane < k ? pos_of[t * k + lane] : -1;
   uint4 out[QT_CPW];
@@ -332,18 +347,18 @@ int moe_permute_impl(int32_t* sorted_pair, int32_t* expert_offsets, const int32_
     attr_done[dev] = true;
   }
   if (P <= kChunk) {
-    permute_small_kernel<<<1, kChunk, smem, st>>>(ids, P, (int)E, expert_offsets, sorted_pair, status, mtiles,
-                                                  num_mtiles, max_mtiles, pos_of, split_cnt);
     if (tiles_done) *tiles_done = mtiles != nullptr;
-    return moe_launch_status();
+    return moe_launch(permute_small_kernel, 1, kChunk, smem, st, ids, P, (int)E, expert_offsets, sorted_pair, status, mtiles,
+                      num_mtiles, max_mtiles, pos_of, split_cnt);
   }
   MOE_CHECK_ARG(scratch);
   const int nchunks = (int)((P + kChunk - 1) / kChunk);
-  permute_hist_kernel<<<nchunks, kChunk, smem, st>>>(ids, P, (int)E, scratch, status);
-  permute_scan_kernel<<<1, kChunk, 0, st>>>(scratch, nchunks, (int)E, expert_offsets);
-  permute_scatter_kernel<<<nchunks, kChunk, smem, st>>>(ids, P, (int)E, scratch, expert_offsets, sorted_pair,
-                                                        pos_of);
-  return moe_launch_status();
+  int rc = moe_launch(permute_hist_kernel, nchunks, kChunk, smem, st, ids, P, (int)E, scratch, status);
+  if (!rc) rc = moe_launch(permute_scan_kernel, 1, kChunk, 0, st, scratch, nchunks, (int)E, expert_offsets);
+  if (!rc)
+    rc = moe_launch(permute_scatter_kernel, nchunks, kChunk, smem, st, ids, P, (int)E, scratch, expert_offsets, sorted_pair,
+                    pos_of);
+  return rc;
 }
 
 extern "C" int b200moe_permute(int32_t* sorted_pair, int32_t* expert_offsets, const int32_t* ids, int64_t T,
@@ -359,9 +374,8 @@ extern "C" int b200moe_gather_scatter_index(int32_t* gather_index, int32_t* scat
   MOE_CHECK_ARG(gather_index && scatter_index && num_per_expert && sorted_pair && expert_offsets);
   MOE_CHECK_ARG(T >= 0 && k > 0 && E > 0);
   if (T == 0) return B200MOE_OK;
-  gather_scatter_index_kernel<<<(unsigned)E, 256, 0, (cudaStream_t)stream>>>(
-      gather_index, scatter_index, num_per_expert, sorted_pair, expert_offsets, T, (int)k);
-  return moe_launch_status();
+  return moe_launch(gather_scatter_index_kernel, (unsigned)E, 256, 0, (cudaStream_t)stream, gather_index, scatter_index,
+                    num_per_expert, sorted_pair, expert_offsets, T, (int)k);
 }
 
 namespace {
@@ -370,9 +384,8 @@ int launch_quant_rows(uint8_t* q, float* s_t, int64_t ld, const void* x, const i
   const int chunks = (int)((H + 255) / 256);
   const int cpw = rows >= 2048 ? chunks : 1;
   const int warps_per_row = (chunks + cpw - 1) / cpw;
-  quant_rows_kernel<<<(unsigned)((rows * warps_per_row + 7) / 8), 256, 0, st>>>(
-      q, s_t, ld, reinterpret_cast<const __nv_bfloat16*>(x), row_map, (int)div, rows, (int)H, cpw, warps_per_row, lists);
-  return moe_launch_status();
+  return moe_launch(quant_rows_kernel, (unsigned)((rows * warps_per_row + 7) / 8), 256, 0, st, q, s_t, ld,
+                    reinterpret_cast<const __nv_bfloat16*>(x), row_map, (int)div, rows, (int)H, cpw, warps_per_row, lists);
 }
 }  // namespace
 
@@ -391,14 +404,13 @@ int moe_quant_identity(uint8_t* q, float* s_t, int64_t ld, const void* x, int64_
 }
 
 int moe_quant_tokens(uint8_t* q, float* s_t, int64_t ld, const void* x, const int32_t* pos_of, int64_t T, int64_t k,
-                     int64_t H, cudaStream_t st) {
+                     int64_t H, float* acc32, cudaStream_t st) {
   const int64_t chunks = (H + 511) / 512;
   // two chunks per warp once that still leaves every SM its full set of warps
   const int cpw = T * chunks >= 2 * 64 * 148 ? QT_CPW : 1;
   const int64_t wpt = (chunks + cpw - 1) / cpw;
-  quant_tokens_kernel<<<(unsigned)((T * wpt + 7) / 8), 256, 0, st>>>(
-      q, s_t, ld, reinterpret_cast<const __nv_bfloat16*>(x), pos_of, T, (int)k, (int)H, cpw, (int)wpt);
-  return moe_launch_status();
+  return moe_launch(quant_tokens_kernel, (unsigned)((T * wpt + 7) / 8), 256, 0, st, q, s_t, ld,
+                    reinterpret_cast<const __nv_bfloat16*>(x), pos_of, T, (int)k, (int)H, cpw, (int)wpt, acc32);
 }
 
 // ---- permutation without caller-provided scratch ---------------------------------------------------

@@ -123,6 +123,7 @@ template <int VPT>
 __global__ void __launch_bounds__(kWarpsPerBlock * 32)
 topk_kernel(void* __restrict__ values, int32_t* __restrict__ indices, const void* __restrict__ scores,
             int dtype, int64_t batch, int n, int n_groups, int topk_groups, int k) {
+  pdl_begin();
   const int lane = threadIdx.x & 31;
   const int64_t row = (int64_t)blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
   if (row >= batch) return;
@@ -147,6 +148,7 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32)
 route_kernel(int32_t* __restrict__ ids, float* __restrict__ w, __nv_bfloat16* __restrict__ w_bf16,
              const float* __restrict__ logits, const float* __restrict__ logit_bias,
              const float* __restrict__ bias, int64_t T, int n, int k, int score_func, int n_groups, int topk_groups, int renorm, float scale) {
+  pdl_begin();
   const int lane = threadIdx.x & 31;
   const int64_t row = (int64_t)blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
   if (row >= T) return;
@@ -250,6 +252,7 @@ __device__ __forceinline__ void cp_async16(void* smem_dst, const void* gsrc, int
 __global__ void __launch_bounds__(RG_THREADS)
 router_gemm_kernel(float* __restrict__ logits, const __nv_bfloat16* __restrict__ x,
                    const __nv_bfloat16* __restrict__ wr, int64_t T, int64_t H, int64_t E) {
+  pdl_begin();
   extern __shared__ __align__(16) uint8_t rg_smem[];
   __nv_bfloat16* const stages = reinterpret_cast<__nv_bfloat16*>(rg_smem);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -363,6 +366,7 @@ constexpr int RV_MAXT = 8;
 __global__ void __launch_bounds__(128)
 router_gemv_kernel(float* __restrict__ logits, const __nv_bfloat16* __restrict__ x,
                    const __nv_bfloat16* __restrict__ wr, int64_t T, int64_t H, int64_t E) {
+  pdl_begin();
   __shared__ float part[4][RV_MAXT];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int64_t e = blockIdx.x;
@@ -409,6 +413,7 @@ template <int EP>
 __global__ void __launch_bounds__(RS_WARPS * 32)
 router_small_e_kernel(float* __restrict__ logits, const __nv_bfloat16* __restrict__ x,
                        const __nv_bfloat16* __restrict__ wr, int64_t T, int64_t H, int E) {
+  pdl_begin();
   __shared__ float part[RS_WARPS][RS_TOK][EP];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int64_t t0 = (int64_t)blockIdx.x * RS_TOK;
@@ -489,9 +494,8 @@ int launch_topk(void* values, int32_t* indices, const void* scores, int dtype, i
   if (batch == 0) return B200MOE_OK;
   dim3 grid((unsigned)((batch + kWarpsPerBlock - 1) / kWarpsPerBlock));
   return dispatch_vpt(n, [&](auto vpt) {
-    topk_kernel<decltype(vpt)::value><<<grid, kWarpsPerBlock * 32, 0, (cudaStream_t)stream>>>(
-        values, indices, scores, dtype, batch, (int)n, (int)n_groups, (int)topk_groups, (int)k);
-    return moe_launch_status();
+    return moe_launch(topk_kernel<decltype(vpt)::value>, grid, kWarpsPerBlock * 32, 0, (cudaStream_t)stream, values, indices,
+                      scores, dtype, batch, (int)n, (int)n_groups, (int)topk_groups, (int)k);
   });
 }
 
@@ -522,10 +526,9 @@ extern "C" int b200moe_route(int32_t* ids, float* w, void* w_bf16, const float* 
   if (T == 0) return B200MOE_OK;
   dim3 grid((unsigned)((T + kWarpsPerBlock - 1) / kWarpsPerBlock));
   return dispatch_vpt(E, [&](auto vpt) {
-    route_kernel<decltype(vpt)::value><<<grid, kWarpsPerBlock * 32, 0, (cudaStream_t)stream>>>(
-        ids, w, reinterpret_cast<__nv_bfloat16*>(w_bf16), logits, logit_bias, bias, T, (int)E, (int)k, score_func,
-        (int)(n_groups > 1 ? n_groups : 1), (int)topk_groups, renorm, scale);
-    return moe_launch_status();
+    return moe_launch(route_kernel<decltype(vpt)::value>, grid, kWarpsPerBlock * 32, 0, (cudaStream_t)stream, ids, w,
+                      reinterpret_cast<__nv_bfloat16*>(w_bf16), logits, logit_bias, bias, T, (int)E, (int)k, score_func,
+                      (int)(n_groups > 1 ? n_groups : 1), (int)topk_groups, renorm, scale);
   });
 }
 
@@ -538,12 +541,11 @@ extern "C" int b200moe_router_logits(float* logits, const void* x, const void* w
   auto xb = reinterpret_cast<const __nv_bfloat16*>(x);
   auto wb = reinterpret_cast<const __nv_bfloat16*>(wr);
   if (T <= 2 * RV_MAXT) {
-    dim3 grid((unsigned)E, (unsigned)((T + RV_MAXT - 1) / RV_MAXT));
-    router_gemv_kernel<<<grid, 128, 0, (cudaStream_t)stream>>>(logits, xb, wb, T, H, E);
+    return moe_launch(router_gemv_kernel, dim3((unsigned)E, (unsigned)((T + RV_MAXT - 1) / RV_MAXT)), 128, 0,
+                      (cudaStream_t)stream, logits, xb, wb, T, H, E);
   } else if (E <= 16) {
-    const unsigned grid = (unsigned)((T + RS_TOK - 1) / RS_TOK);
-    if (E <= 8) router_small_e_kernel<8><<<grid, RS_WARPS * 32, 0, (cudaStream_t)stream>>>(logits, xb, wb, T, H, (int)E);
-    else router_small_e_kernel<16><<<grid, RS_WARPS * 32, 0, (cudaStream_t)stream>>>(logits, xb, wb, T, H, (int)E);
+    return moe_launch(E <= 8 ? router_small_e_kernel<8> : router_small_e_kernel<16>, dim3((unsigned)((T + RS_TOK - 1) / RS_TOK)),
+                      RS_WARPS * 32, 0, (cudaStream_t)stream, logits, xb, wb, T, H, (int)E);
   } else {
     constexpr int kMaxDevices = 64;
     static bool attr_done[kMaxDevices] = {};
@@ -556,19 +558,7 @@ extern "C" int b200moe_router_logits(float* logits, const void* x, const void* w
     const int64_t mt = (T + RG_BM - 1) / RG_BM, nt = (E + RG_BN - 1) / RG_BN;
     int splits = 1;  // as many as there are SMs for, with at least 256 columns of K each
     while (splits < RG_MAX_SPLIT && mt * nt * splits * 2 <= moe_device_sm_count() && H / (splits * 2) >= 4 * RG_BK) splits *= 2;
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3((unsigned)mt, (unsigned)splits, (unsigned)nt);
-    cfg.blockDim = dim3(RG_THREADS);
-    cfg.dynamicSmemBytes = RG_SMEM_BYTES;
-    cfg.stream = (cudaStream_t)stream;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = at[0].val.clusterDim.z = 1;
-    at[0].val.clusterDim.y = (unsigned)splits;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    const cudaError_t e = cudaLaunchKernelEx(&cfg, router_gemm_kernel, logits, xb, wb, T, H, E);
-    if (e != cudaSuccess) return (int)e;
+    return moe_launch_cluster(splits, router_gemm_kernel, dim3((unsigned)mt, (unsigned)splits, (unsigned)nt), RG_THREADS,
+                              RG_SMEM_BYTES, (cudaStream_t)stream, logits, xb, wb, T, H, E);
   }
-  return moe_launch_status();
 }
