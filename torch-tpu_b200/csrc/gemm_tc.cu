@@ -10,9 +10,9 @@
 //          the rank that owns the token (expert parallelism over peer memory: plain peer stores)
 //   linear out = x W^T with W [N,K]      one "expert", no activation, bf16 rows out (my_ops/MmW8A16Dq.cpp:185-229)
 //
-// One persistent CTA per SM, 12 warps: warp 0 = TMA producer, warp 1 = MMA issuer (one thread) and TMEM
+// One persistent CTA per SM, 12 warps: warp 0 = TMA producer of the weights, warp 1 = MMA issuer (one thread) and TMEM
 // owner, warp 2 = scout (walks the next work item's expert, row range and first scales and leaves them in shared
-// memory), warp 3 idle, warps 4..11 = epilogue (TMEM lane quarter = warp%4, column half = (warp-4)/4).  setmaxnreg
+// memory), warp 3 = TMA producer of the activations, warps 4..11 = epilogue (TMEM lane quarter = warp%4, column half = (warp-4)/4).  setmaxnreg
 // moves registers from the first warpgroup to the epilogue.  Results leave through shared memory: every epilogue warp
 // turns its 32 rows x 64 columns through a private patch and stores whole 64- or 128-byte row segments.
 // A tile is 128 rows x 256 MMA columns: gemm1 -> 128 gate + 128 up columns of one 128-wide slice of I
@@ -22,6 +22,8 @@
 //
 // No multicast loads anywhere.  Every wait is bounded: on a time-out the CTA raises status bit 1, all roles
 // leave their loops, tensor memory is released and the kernel returns.
+#include <type_traits>
+
 #include "schedule.h"
 #include "tc_ptx.cuh"
 
@@ -36,7 +38,7 @@ constexpr int TC_CH = 16;                    // columns per tcgen05.ld (= regist
 constexpr int TC_CPH = TC_CW / TC_CH;        // TMEM chunks per half
 constexpr int TC_NC = 2 * TC_CPH;            // chunks per thread and K block
 constexpr int TC_EPI_THREADS = 128 * TC_CG;
-constexpr int TC_THREADS = 128 + TC_EPI_THREADS;  // warpgroup 0 = {producer, MMA, scout, idle}, then the epilogue warps
+constexpr int TC_THREADS = 128 + TC_EPI_THREADS;  // warpgroup 0 = {B producer, MMA, scout, A producer}, then the epilogue warps
 // setmaxnreg targets: warpgroup 0 gives registers to the epilogue.  The increase blocks until the CTA's pool (the
 // launch-time count x threads) holds enough, so 128 * LO + TC_EPI_THREADS * HI must not exceed that pool:
 // 384 threads x 168 = 128 x 72 + 256 x 216; 640 threads x 96 = 128 x 32 + 512 x 112.
@@ -50,6 +52,8 @@ static_assert(128 * TC_REG_LO + TC_EPI_THREADS * TC_REG_HI <= TC_THREADS * TC_RE
               "setmaxnreg.inc would wait for registers that the CTA's pool never holds");
 constexpr int TC_STAGES = 4;
 constexpr int TC_A_BYTES = 128 * 128;       // 128 rows x 128 B
+constexpr int TC_AR = 16;                   // rows of the small A box ...
+constexpr int TC_AR_BYTES = TC_AR * 128;    // ... which brings just the rows that a short tile has
 constexpr int TC_B_BYTES = 2 * 128 * 128;   // two 128 x 128 B boxes
 constexpr int TC_STAGE_BYTES = TC_A_BYTES + TC_B_BYTES;
 constexpr int TC_TMEM_COLS = 512;           // two accumulator buffers of 256 fp32 columns
@@ -139,8 +143,8 @@ __host__ __device__ constexpr uint32_t make_idesc(int b_mn_major) {
 // W [N, K] K-major (the gate/up operand path with the down GEMM's bf16 store; a.I = N, a.H = K, 256 outputs per tile)
 template <int MODE>
 __global__ void __launch_bounds__(TC_THREADS, 1)
-moe_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB0,
-                   const __grid_constant__ CUtensorMap tmB1, const TcArgs a) {
+moe_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmAs,
+                   const __grid_constant__ CUtensorMap tmB0, const __grid_constant__ CUtensorMap tmB1, const TcArgs a) {
   constexpr bool GEMM2 = MODE == 1, DENSE = MODE == 2;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -151,7 +155,7 @@ moe_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < TC_STAGES; ++s) {
-      mbar_init(smem_u32(&sh->full[s]), 1);
+      mbar_init(smem_u32(&sh->full[s]), 2);  // the two producers
       mbar_init(smem_u32(&sh->empty[s]), 1);
     }
     for (int b = 0; b < 2; ++b) {
@@ -170,12 +174,20 @@ moe_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
+  // The A stages start as zeros.  A tile of at most 32 rows loads only the one or two 16-row boxes it needs, so the other
+  // rows of its MMAs multiply zeros (or an earlier tile's rows) instead of the next experts' rows: this part runs at its
+  // power limit even where it only streams weights, and the tensor cores' switching on rows nobody asked for came out of
+  // the clock (DeepSeek shape, 64 tokens: 1410 -> 1530 MHz, layer 1.78 -> 1.64 ms; Mixtral shape, 1 token: 106 -> 95 us).
+  // Taller tiles take the one 128-row box: four or more small boxes per K block cost more than they saved (DeepSeek
+  // shape, 2048 tokens, 64 rows per expert: 2.60 -> 2.70 ms).
+  for (int i = threadIdx.x; i < TC_STAGES * (TC_A_BYTES / 16); i += TC_THREADS)
+    *reinterpret_cast<uint4*>(smem + (i / (TC_A_BYTES / 16)) * TC_STAGE_BYTES + (i % (TC_A_BYTES / 16)) * 16) = make_uint4(0, 0, 0, 0);
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = sh->tmem_base;
-  // Everything above overlaps the end of the kernel before this one.  Where the work list is older than that kernel, the
-  // producer also requests its first weight tiles before the wait (they are nobody's output).
+  // Everything above overlaps the end of the kernel before this one.
   if (!a.lists_ready) pdl_wait();
 
   const int num_mtiles = *a.num_mtiles;
@@ -221,66 +233,43 @@ moe_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
   const bool rows_out = MODE != 0 && (a.row_src || (a.KS == 1 && !a.comb32 && !(DENSE && a.out32)));
   if (warp < 4) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(TC_REG_LO));
   if (warp == 0) {
-    // ------------------------------------------------------------------ TMA producer (one thread)
+    // ------------------------------------------------------------------ TMA producer of the weights (one thread)
+    // Two producers, this one for B and warp 3's for A, each on its own clock.  Weights are nobody's output: where the
+    // work list is ready they are requested before the kernel in front of this one has finished.
     if (lane == 0) {
-      uint32_t it = 0;
       bool ok = true;
       // the m-tile list entry of the NEXT work item is requested while this one's loads are issued: when the weights
       // stream from HBM the ring is empty at every tile start, and a dependent L2 round trip there is pure idle time
       Item nx{};
-      int nx_e = 0, nx_row0 = 0;
+      int nx_e = 0;
       if ((int)blockIdx.x < total_tiles) {
         nx = item_of(blockIdx.x);
-        nx_e = a.mtiles[2 * nx.mt], nx_row0 = a.mtiles[2 * nx.mt + 1];
+        nx_e = a.mtiles[2 * nx.mt];
       }
-      auto load_b = [&](int nt, int e, int kb, uint32_t sb, uint32_t full) {
-        if (DENSE) {
-          tma_load_2d(sb, &tmB0, kb * kBlock, e * a.I + nt * 256, full);
-          tma_load_2d(sb + 128 * 128, &tmB0, kb * kBlock, e * a.I + nt * 256 + 128, full);
-        } else if (!GEMM2) {
-          tma_load_2d(sb, &tmB0, kb * kBlock, e * a.I + nt * 128, full);
-          tma_load_2d(sb + 128 * 128, &tmB1, kb * kBlock, e * a.I + nt * 128, full);
-        } else {
-          tma_load_2d(sb, &tmB0, nt * 256, e * a.I + kb * kBlock, full);
-          tma_load_2d(sb + 128 * 128, &tmB0, nt * 256 + 128, e * a.I + kb * kBlock, full);
-        }
-      };
-      // the first item's first weight tiles; their A tiles follow after the wait (the ring is empty: no stage to wait for)
-      uint32_t n_early = 0;
-      if (a.lists_ready) {
-        if ((int)blockIdx.x < total_tiles) {
-          n_early = nx.KB < TC_STAGES ? nx.KB : TC_STAGES;
-          for (uint32_t s = 0; s < n_early; ++s) {
-            const uint32_t full = smem_u32(&sh->full[s]);
-            mbar_arrive_expect_tx(full, TC_STAGE_BYTES);
-            load_b(nx.nt, nx_e, nx.kb0 + s, smem_base + s * TC_STAGE_BYTES + TC_A_BYTES, full);
-          }
-        }
-        pdl_wait();
-      }
+      uint32_t s = 0, ph = 1;
       for (int t = blockIdx.x; t < total_tiles && ok; t += gridDim.x) {
-        const int nt = nx.nt, kb0 = nx.kb0, kb1 = nx.kb0 + nx.KB;
-        const int e = nx_e, row0 = nx_row0;
+        const int KB = nx.KB;
+        // coordinates of the two boxes of the first K block, and their step per K block
+        const int n0 = nx_e * a.I + (GEMM2 ? nx.kb0 * kBlock : nx.nt * (DENSE ? 256 : 128));  // row of the weight matrix
+        const int c0 = GEMM2 ? nx.nt * 256 : nx.kb0 * kBlock;
         if (t + (int)gridDim.x < total_tiles) {
           nx = item_of(t + gridDim.x);
-          nx_e = a.mtiles[2 * nx.mt], nx_row0 = a.mtiles[2 * nx.mt + 1];
+          nx_e = a.mtiles[2 * nx.mt];
         }
-        for (int kb = kb0; kb < kb1; ++kb, ++it) {
-          const int s = it % TC_STAGES;
-          const uint32_t ph = (it / TC_STAGES) & 1;
-          const uint32_t full = smem_u32(&sh->full[s]);
-          const uint32_t sa = smem_base + s * TC_STAGE_BYTES, sb = sa + TC_A_BYTES;
-          if (it < n_early) {
-            tma_load_2d(sa, &tmA, kb * kBlock, row0, full);
-            continue;
-          }
-          if (!mbar_wait(smem_u32(&sh->empty[s]), ph ^ 1, abort_flag)) {
+        int row = n0, col = c0;
+        for (int kb = 0; kb < KB; ++kb) {
+          const uint32_t full = smem_u32(&sh->full[0]) + s * 8, sb = smem_base + TC_A_BYTES + s * TC_STAGE_BYTES;
+          if (!mbar_wait(smem_u32(&sh->empty[0]) + s * 8, ph, abort_flag)) {
             ok = false;
             break;
           }
-          mbar_arrive_expect_tx(full, TC_STAGE_BYTES);
-          tma_load_2d(sa, &tmA, kb * kBlock, row0, full);
-          load_b(nt, e, kb, sb, full);
+          mbar_arrive_expect_tx(full, TC_B_BYTES);
+          tma_load_2d(sb, &tmB0, col, row, full);
+          if (GEMM2) tma_load_2d(sb + 128 * 128, &tmB0, col + 128, row, full);
+          else tma_load_2d(sb + 128 * 128, DENSE ? &tmB0 : &tmB1, col, row + (DENSE ? 128 : 0), full);
+          if (GEMM2) row += kBlock;
+          else col += kBlock;
+          if (++s == TC_STAGES) s = 0, ph ^= 1;
         }
       }
     }
@@ -381,7 +370,43 @@ moe_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
       }
     }
   } else if (warp == 3) {
-    pdl_begin();  // let the next kernel's CTAs come up as this one's leave
+    // ------------------------------------------------------------------ TMA producer of the activations (one thread)
+    pdl_begin();  // (also lets the next kernel's CTAs come up as this one's leave)
+    if (lane == 0) {
+      bool ok = true;
+      Item nx{};
+      int nx_row0 = 0, nx_end = 0;
+      auto fetch = [&](int t) {
+        nx = item_of(t);
+        nx_row0 = a.mtiles[2 * nx.mt + 1];
+        nx_end = a.offsets[a.mtiles[2 * nx.mt] + 1];
+      };
+      if ((int)blockIdx.x < total_tiles) fetch(blockIdx.x);
+      uint32_t s = 0, ph = 1;
+      for (int t = blockIdx.x; t < total_tiles && ok; t += gridDim.x) {
+        const int KB = nx.KB, row0 = nx_row0, n = (min(nx_end, a.P) - nx_row0 + TC_AR - 1) / TC_AR;
+        int col = nx.kb0 * kBlock;
+        if (t + (int)gridDim.x < total_tiles) fetch(t + gridDim.x);
+        auto k_loop = [&](auto boxes) {  // small A boxes of the tile; 0 = the one 128-row box
+          constexpr int BOXES = decltype(boxes)::value;
+          for (int kb = 0; kb < KB; ++kb) {
+            const uint32_t full = smem_u32(&sh->full[0]) + s * 8, sa = smem_base + s * TC_STAGE_BYTES;
+            if (!mbar_wait(smem_u32(&sh->empty[0]) + s * 8, ph, abort_flag)) {
+              ok = false;
+              break;
+            }
+            mbar_arrive_expect_tx(full, BOXES ? BOXES * TC_AR_BYTES : TC_A_BYTES);
+            tma_load_2d(sa, BOXES ? &tmAs : &tmA, col, row0, full);
+            if (BOXES == 2) tma_load_2d(sa + TC_AR_BYTES, &tmAs, col, row0 + TC_AR, full);
+            col += kBlock;
+            if (++s == TC_STAGES) s = 0, ph ^= 1;
+          }
+        };
+        if (n > 2) k_loop(std::integral_constant<int, 0>{});
+        else if (n == 2) k_loop(std::integral_constant<int, 2>{});
+        else k_loop(std::integral_constant<int, 1>{});
+      }
+    }
   } else if (warp >= 4) {
     pdl_wait();
     // ------------------------------------------------------------------ epilogue (4 * TC_CG warps)
@@ -603,7 +628,8 @@ moe_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
       // lane into 32 different rows per instruction: half-used sectors (and, to a peer, 32 small packets), which cost
       // several thousand cycles per tile.  Each warp turns its own 32 rows x TC_CW columns through a private patch of
       // shared memory instead (16-byte chunks, XOR-swizzled so that neither side has bank conflicts; only warp-level
-      // synchronisation) and then stores whole 64- or 128-byte row segments per group of lanes.
+      // synchronisation) and then stores whole 64- or 128-byte row segments per group of lanes.  (Handing each row's
+      // 128 bytes to the copy engine, so that the warp could go on, was slower: Qwen3 down GEMM 217 -> 241 us.)
       static_assert(TC_CW == 64, "the row-segment stores below are laid out for 64 columns per warp");
       const int wepi = warp - 4;
       if (MODE == 0) {
@@ -741,13 +767,13 @@ moe_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
 }
 
 // ---- host side ---------------------------------------------------------------------------------------
-// row-major u8 matrix [rows, cols], box 128 x 128 bytes, 128-byte swizzle, zero fill outside
-bool make_map_u8(CUtensorMap* m, const void* base, uint64_t rows, uint64_t cols) {
+// row-major u8 matrix [rows, cols], box `box_rows` x 128 bytes, 128-byte swizzle, zero fill outside
+bool make_map_u8(CUtensorMap* m, const void* base, uint64_t rows, uint64_t cols, uint32_t box_rows = 128) {
   EncodeTiledFn enc = get_encode_fn();
   if (!enc) return false;
   cuuint64_t dims[2] = {cols, rows};
   cuuint64_t strides[1] = {cols};
-  cuuint32_t box[2] = {128, 128};
+  cuuint32_t box[2] = {128, box_rows};
   cuuint32_t es[2] = {1, 1};
   return enc(m, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void*>(base), dims, strides, box, es,
              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
@@ -787,8 +813,9 @@ int launch_tc(const MoeGemmArgs& g, cudaStream_t st) {
   if (g.scale_dtype != B200MOE_F32) return B200MOE_EINVAL;  // the caller converts bf16 scales first
   if ((int64_t)g.E * ((g.I + kBlock - 1) / kBlock) * (g.H / kBlock) >= (int64_t(1) << 31)) return B200MOE_EINVAL;  // 32-bit scale indices
   const int K = GEMM2 ? g.I : g.H;
-  CUtensorMap tmA, tmB0, tmB1;
+  CUtensorMap tmA, tmAs, tmB0, tmB1;
   if (!make_map_u8(&tmA, g.aq, (uint64_t)g.P, (uint64_t)K)) return B200MOE_EDRIVER;
+  if (!make_map_u8(&tmAs, g.aq, (uint64_t)g.P, (uint64_t)K, TC_AR)) return B200MOE_EDRIVER;
   if (!make_map_u8(&tmB0, g.w0, (uint64_t)g.E * g.I, (uint64_t)g.H)) return B200MOE_EDRIVER;
   if (!make_map_u8(&tmB1, (GEMM2 || DENSE) ? g.w0 : g.w1, (uint64_t)g.E * g.I, (uint64_t)g.H)) return B200MOE_EDRIVER;
   TcArgs a{};
@@ -849,7 +876,7 @@ int launch_tc(const MoeGemmArgs& g, cudaStream_t st) {
   const int grid = (int)((a.part ? max_tiles * kMaxParts : max_tiles) < sms ? (a.part ? max_tiles * kMaxParts : max_tiles) : sms);
   if (grid > kMaxSplitCtas) a.part = nullptr;  // the slots are laid out for that many
   a.lists_ready = g.lists_ready;
-  return moe_launch(moe_gemm_tc_kernel<MODE>, grid, TC_THREADS, TC_SMEM_BYTES, st, tmA, tmB0, tmB1, a);
+  return moe_launch(moe_gemm_tc_kernel<MODE>, grid, TC_THREADS, TC_SMEM_BYTES, st, tmA, tmAs, tmB0, tmB1, a);
 }
 
 }  // namespace
