@@ -235,14 +235,9 @@ extern "C" int b200moe_experts(void* out, const void* x, const void* w_gate, con
   }
 
   if (do_prep) {
-    bool tiles_done = false;
     rc = moe_permute_impl(I32(L.sorted), I32(L.offsets), ids, d->T, d->k, d->E, I32(L.scratch), status, I32(L.pos_of),
-                          I32(L.mtiles), I32(L.nmt), L.max_mtiles, I32(L.cnt), &tiles_done, stream);
+                          I32(L.mtiles), I32(L.nmt), L.max_mtiles, I32(L.cnt), stream);
     if (rc) return rc;
-    if (!tiles_done) {
-      rc = moe_build_mtiles(I32(L.mtiles), I32(L.nmt), I32(L.offsets), (int)d->E, L.P, L.max_mtiles, I32(L.cnt), st);
-      if (rc) return rc;
-    }
   }
   if (w8a8 && do_prep) {
     rc = moe_quant_tokens(reinterpret_cast<uint8_t*>(ws + L.xq), reinterpret_cast<float*>(ws + L.xs), L.ld, x,

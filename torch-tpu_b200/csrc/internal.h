@@ -85,10 +85,10 @@ __device__ __forceinline__ void moe_write_identity_lists(const MoeIdentityLists&
 }
 #endif
 
-// b200moe_permute that also writes the inverse map (pos_of, may be NULL) and the m-tile list when one CTA does the whole sort (at most 1024 pairs)
+// b200moe_permute that also writes the inverse map (pos_of, may be NULL) and the m-tile list (mtiles, may be NULL)
 int moe_permute_impl(int32_t* sorted_pair, int32_t* expert_offsets, const int32_t* ids, int64_t T, int64_t k, int64_t E,
                      int32_t* scratch, int32_t* status, int32_t* pos_of, int32_t* mtiles, int32_t* num_mtiles,
-                     int max_mtiles, int32_t* split_cnt, bool* tiles_done, void* stream);
+                     int max_mtiles, int32_t* split_cnt, void* stream);
 // quantised rows of x at the positions of every token's k pairs (and zeros to acc32 [T,H], may be NULL); quantised rows 0..rows with the identity lists
 int moe_quant_tokens(uint8_t* q, float* s_t, int64_t ld, const void* x, const int32_t* pos_of, int64_t T, int64_t k,
                      int64_t H, float* acc32, cudaStream_t st);

@@ -7,7 +7,7 @@
 //   scan    : per expert a running sum over chunks, then a scan over experts -> chunk_base, offsets
 //   scatter : position = offsets[e] + chunk_base[c][e] + (pairs of e in earlier warps of the chunk)
 //             + (pairs of e in lower lanes of the warp)
-// For P <= 1024 all three steps run in one single-CTA kernel.
+// For P <= 1024 all three steps run in one single-CTA kernel, up to 8192 in one cluster of CTAs.
 #include "internal.h"
 
 namespace {
@@ -53,25 +53,47 @@ permute_hist_kernel(const int32_t* __restrict__ ids, int64_t P, int E, int32_t* 
   }
 }
 
-// exclusive scan of cnt[0..E) by one CTA of 1024 threads (E <= 1024); result in offs[0..E], smem tmp[1024]
-__device__ __forceinline__ void block_exclusive_scan(int my, int E, int32_t* __restrict__ offs, int* tmp) {
-  const int t = threadIdx.x;
-  tmp[t] = t < E ? my : 0;
-  __syncthreads();
-  for (int d = 1; d < kChunk; d <<= 1) {
-    int v = t >= d ? tmp[t - d] : 0;
-    __syncthreads();
-    tmp[t] += v;
-    __syncthreads();
+// exclusive scan of the threads' counts (thread t < E: expert t) by one CTA of 1024 threads; result in offs[0..E], valid
+// after the next __syncthreads
+__device__ __forceinline__ void block_exclusive_scan(int my, int E, int32_t* offs, int* tmp /* [32] */) {
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  int v = t < E ? my : 0;
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const int u = __shfl_up_sync(0xffffffffu, v, d);
+    if (lane >= d) v += u;
   }
-  if (t < E) offs[t + 1] = tmp[t];
+  __syncthreads();  // tmp of the scan before is read
+  if (lane == 31) tmp[warp] = v;
+  __syncthreads();
+  int before = 0;
+  for (int w = 0; w < warp; ++w) before += tmp[w];
+  if (t < E) offs[t + 1] = before + v;
   if (t == 0) offs[0] = 0;
 }
 
+// what the grouped GEMMs walk, written by one CTA from the expert offsets in shared memory: {expert, first row} per 128
+// rows of an expert, their number, and zeros in the counters of shared tiles
+__device__ __forceinline__ void write_mtiles(const int* soffs, int E, int* toffs, int* tmp, int32_t* __restrict__ mtiles,
+                                             int32_t* __restrict__ num_mtiles, int max_mtiles, int32_t* split_cnt) {
+  moe_clear_counters(split_cnt);
+  const int t = threadIdx.x;
+  const int b = t < E ? soffs[t] : 0;
+  const int n = t < E ? (soffs[t + 1] - b + kTileM - 1) / kTileM : 0;
+  block_exclusive_scan(n, E, toffs, tmp);
+  __syncthreads();
+  for (int i = 0; i < n && toffs[t] + i < max_mtiles; ++i) {
+    mtiles[2 * (toffs[t] + i)] = t;
+    mtiles[2 * (toffs[t] + i) + 1] = b + i * kTileM;
+  }
+  if (t == 0) *num_mtiles = min(toffs[E], max_mtiles);
+}
+
 __global__ void __launch_bounds__(kChunk)
-permute_scan_kernel(int32_t* __restrict__ chunk_cnt, int nchunks, int E, int32_t* __restrict__ offsets) {
+permute_scan_kernel(int32_t* __restrict__ chunk_cnt, int nchunks, int E, int32_t* __restrict__ offsets,
+                    int32_t* __restrict__ mtiles, int32_t* __restrict__ num_mtiles, int max_mtiles, int32_t* split_cnt) {
   pdl_begin();
-  __shared__ int tmp[kChunk];
+  __shared__ int tmp[32], soffs[kMaxE + 1], toffs[kMaxE + 1];
   int total = 0;
   if ((int)threadIdx.x < E) {
     // eight counts are requested before the first is used: walked one by one, every chunk costs an L2 round trip
@@ -87,7 +109,10 @@ permute_scan_kernel(int32_t* __restrict__ chunk_cnt, int nchunks, int E, int32_t
       }
     }
   }
-  block_exclusive_scan(total, E, offsets, tmp);
+  block_exclusive_scan(total, E, soffs, tmp);
+  __syncthreads();
+  for (int i = threadIdx.x; i <= E; i += blockDim.x) offsets[i] = soffs[i];
+  if (mtiles) write_mtiles(soffs, E, toffs, tmp, mtiles, num_mtiles, max_mtiles, split_cnt);
 }
 
 __global__ void __launch_bounds__(kChunk)
@@ -128,8 +153,7 @@ permute_small_kernel(const int32_t* __restrict__ ids, int64_t P, int E, int32_t*
                      int32_t* split_cnt) {
   pdl_begin();
   extern __shared__ int wh[];
-  __shared__ int tmp[kChunk];
-  __shared__ int soffs[kMaxE + 1];
+  __shared__ int tmp[32], soffs[kMaxE + 1], toffs[kMaxE + 1];
   int rank;
   int e = chunk_hist(ids, P, E, threadIdx.x, wh, rank, status);
   int total = 0;
@@ -151,23 +175,65 @@ permute_small_kernel(const int32_t* __restrict__ ids, int64_t P, int E, int32_t*
   }
   if (pos_of && (int64_t)threadIdx.x < P) pos_of[threadIdx.x] = pos;
   if ((int64_t)threadIdx.x < P && (int)threadIdx.x >= soffs[E]) sorted_pair[threadIdx.x] = -1;  // dropped pairs: see above
-  if (mtiles) {
-    // the m-tile list of the grouped GEMMs ({expert, first row} per 128 rows of an expert) from the same offsets:
-    // one launch less on the decode path
-    moe_clear_counters(split_cnt);
-    __syncthreads();
-    const int t = threadIdx.x;
-    const int b = t < E ? soffs[t] : 0;
-    const int n = t < E ? (soffs[t + 1] - b + kTileM - 1) / kTileM : 0;
-    __shared__ int toffs[kMaxE + 1];
-    block_exclusive_scan(n, E, toffs, tmp);
-    __syncthreads();
-    for (int i = 0; i < n && toffs[t] + i < max_mtiles; ++i) {
-      mtiles[2 * (toffs[t] + i)] = t;
-      mtiles[2 * (toffs[t] + i) + 1] = b + i * kTileM;
+  if (mtiles) write_mtiles(soffs, E, toffs, tmp, mtiles, num_mtiles, max_mtiles, split_cnt);
+}
+
+// 1024 < P <= 8192: the same with one cluster, a chunk of 1024 pairs per CTA; the CTAs read one another's counts through
+// distributed shared memory (one launch instead of the three of the general form)
+constexpr int kMaxCluster = 8;  // portable cluster size
+__global__ void __launch_bounds__(kChunk)
+permute_cluster_kernel(const int32_t* __restrict__ ids, int64_t P, int E, int32_t* __restrict__ offsets,
+                       int32_t* __restrict__ sorted_pair, int32_t* status, int32_t* __restrict__ mtiles,
+                       int32_t* __restrict__ num_mtiles, int max_mtiles, int32_t* __restrict__ pos_of, int32_t* split_cnt) {
+  pdl_begin();
+  extern __shared__ int wh[];
+  __shared__ int tmp[32], soffs[kMaxE + 1], toffs[kMaxE + 1], cnt[kMaxE], base[kMaxE];
+  const int me = blockIdx.y, chunks = gridDim.y, t = threadIdx.x;
+  const int64_t p = (int64_t)me * kChunk + t;
+  int rank;
+  const int e = chunk_hist(ids, P, E, p, wh, rank, status);
+  if (t < E) {
+    int total = 0;
+#pragma unroll 8
+    for (int w = 0; w < 32; ++w) {
+      int v = wh[w * E + t];
+      wh[w * E + t] = total;
+      total += v;
     }
-    if (t == 0) *num_mtiles = min(toffs[E], max_mtiles);
+    cnt[t] = total;
   }
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+  int total = 0;
+  if (t < E) {
+    const uint32_t addr = (uint32_t)__cvta_generic_to_shared(cnt + t);
+    int before = 0;
+    for (int c = 0; c < chunks; ++c) {
+      uint32_t remote;
+      int v;
+      asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(addr), "r"(c));
+      asm volatile("ld.shared::cluster.s32 %0, [%1];" : "=r"(v) : "r"(remote) : "memory");
+      if (c < me) before += v;
+      total += v;
+    }
+    base[t] = before;
+  }
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");  // done with the others' counts
+  block_exclusive_scan(total, E, soffs, tmp);
+  __syncthreads();
+  int pos = -1;
+  if (e >= 0) {
+    pos = soffs[e] + base[e] + wh[(t >> 5) * E + e] + rank;
+    sorted_pair[pos] = (int32_t)p;
+  }
+  if (p < P) {
+    if (pos_of) pos_of[p] = pos;
+    if (p >= soffs[E]) sorted_pair[p] = -1;  // dropped pairs: see above
+  }
+  if (me == 0) {
+    for (int i = t; i <= E; i += blockDim.x) offsets[i] = soffs[i];
+    if (mtiles) write_mtiles(soffs, E, toffs, tmp, mtiles, num_mtiles, max_mtiles, split_cnt);
+  }
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");  // nobody leaves while its counts are read
 }
 
 __global__ void gather_scatter_index_kernel(int32_t* __restrict__ gather_index,
@@ -325,12 +391,11 @@ extern "C" size_t b200moe_permute_scratch_ints(int64_t P, int64_t E) {
   return (size_t)((P + kChunk - 1) / kChunk) * (size_t)E;
 }
 
-// b200moe_permute; with `pos_of` != NULL the inverse map too (pos_of[pair] = its position, -1 = dropped); with `mtiles` != NULL and at most 1024 pairs the one-CTA kernel writes the GEMMs' m-tile list too and
-// *tiles_done is set (else the caller builds the list from expert_offsets)
+// b200moe_permute; with `pos_of` != NULL the inverse map too (pos_of[pair] = its position, -1 = dropped); with `mtiles` != NULL the
+// GEMMs' m-tile list too
 int moe_permute_impl(int32_t* sorted_pair, int32_t* expert_offsets, const int32_t* ids, int64_t T, int64_t k, int64_t E,
                      int32_t* scratch, int32_t* status, int32_t* pos_of, int32_t* mtiles, int32_t* num_mtiles,
-                     int max_mtiles, int32_t* split_cnt, bool* tiles_done, void* stream) {
-  if (tiles_done) *tiles_done = false;
+                     int max_mtiles, int32_t* split_cnt, void* stream) {
   MOE_CHECK_ARG(sorted_pair && expert_offsets && ids && T >= 0 && k > 0 && E > 0);
   const int64_t P = T * k;
   MOE_CHECK_SHAPE(E <= kMaxE && P < (1 << 24));
@@ -343,18 +408,22 @@ int moe_permute_impl(int32_t* sorted_pair, int32_t* expert_offsets, const int32_
   if (!attr_done[dev]) {
     cudaFuncSetAttribute(permute_hist_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 32 * kMaxE * 4);
     cudaFuncSetAttribute(permute_scatter_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 32 * kMaxE * 4);
+    cudaFuncSetAttribute(permute_cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 32 * kMaxE * 4);
     cudaFuncSetAttribute(permute_small_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 32 * kMaxE * 4);
     attr_done[dev] = true;
   }
   if (P <= kChunk) {
-    if (tiles_done) *tiles_done = mtiles != nullptr;
     return moe_launch(permute_small_kernel, 1, kChunk, smem, st, ids, P, (int)E, expert_offsets, sorted_pair, status, mtiles,
                       num_mtiles, max_mtiles, pos_of, split_cnt);
   }
   MOE_CHECK_ARG(scratch);
   const int nchunks = (int)((P + kChunk - 1) / kChunk);
+  if (nchunks <= kMaxCluster)
+    return moe_launch_cluster(nchunks, permute_cluster_kernel, dim3(1, nchunks), kChunk, smem, st, ids, P, (int)E,
+                              expert_offsets, sorted_pair, status, mtiles, num_mtiles, max_mtiles, pos_of, split_cnt);
   int rc = moe_launch(permute_hist_kernel, nchunks, kChunk, smem, st, ids, P, (int)E, scratch, status);
-  if (!rc) rc = moe_launch(permute_scan_kernel, 1, kChunk, 0, st, scratch, nchunks, (int)E, expert_offsets);
+  if (!rc) rc = moe_launch(permute_scan_kernel, 1, kChunk, 0, st, scratch, nchunks, (int)E, expert_offsets, mtiles, num_mtiles,
+                            max_mtiles, split_cnt);
   if (!rc)
     rc = moe_launch(permute_scatter_kernel, nchunks, kChunk, smem, st, ids, P, (int)E, scratch, expert_offsets, sorted_pair,
                     pos_of);
@@ -364,7 +433,7 @@ int moe_permute_impl(int32_t* sorted_pair, int32_t* expert_offsets, const int32_
 extern "C" int b200moe_permute(int32_t* sorted_pair, int32_t* expert_offsets, const int32_t* ids, int64_t T,
                                int64_t k, int64_t E, int32_t* scratch, int32_t* status, void* stream) {
   return moe_permute_impl(sorted_pair, expert_offsets, ids, T, k, E, scratch, status, nullptr, nullptr, nullptr, 0,
-                          nullptr, nullptr, stream);
+                          nullptr, stream);
 }
 
 extern "C" int b200moe_gather_scatter_index(int32_t* gather_index, int32_t* scatter_index,
