@@ -143,23 +143,27 @@ topk_kernel(void* __restrict__ values, int32_t* __restrict__ indices, const void
   }
 }
 
+struct RouteArgs {
+  int32_t* ids;
+  float* w;
+  __nv_bfloat16* w_bf16;
+  const float* logit_bias;
+  const float* bias;
+  int k, score_func, n_groups, topk_groups, renorm;
+  float scale;
+};
+
+// One row by one warp: s[j] = logit of element lane + 32*j (elements >= n are not candidates).
 template <int VPT>
-__global__ void __launch_bounds__(kWarpsPerBlock * 32)
-route_kernel(int32_t* __restrict__ ids, float* __restrict__ w, __nv_bfloat16* __restrict__ w_bf16,
-             const float* __restrict__ logits, const float* __restrict__ logit_bias,
-             const float* __restrict__ bias, int64_t T, int n, int k, int score_func, int n_groups, int topk_groups, int renorm, float scale) {
-  pdl_begin();
-  const int lane = threadIdx.x & 31;
-  const int64_t row = (int64_t)blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
-  if (row >= T) return;
-  float s[VPT];    // un-biased scores
-  float sel[VPT];  // selection scores
+__device__ __forceinline__ void route_row(float (&s)[VPT], const RouteArgs& a, int64_t row, int n, int lane) {
+  const int k = a.k;
+  float sel[VPT];  // selection scores; s becomes the un-biased scores
 #pragma unroll
   for (int j = 0; j < VPT; ++j) {
     int e = lane + 32 * j;
-    s[j] = e < n ? (logit_bias ? logits[row * n + e] + logit_bias[e] : logits[row * n + e]) : -INFINITY;
+    s[j] = e < n ? (a.logit_bias ? s[j] + a.logit_bias[e] : s[j]) : -INFINITY;
   }
-  if (score_func == B200MOE_SCORE_SOFTMAX) {
+  if (a.score_func == B200MOE_SCORE_SOFTMAX) {
     float m = -INFINITY;
 #pragma unroll
     for (int j = 0; j < VPT; ++j) m = fmaxf(m, s[j]);
@@ -183,9 +187,9 @@ route_kernel(int32_t* __restrict__ ids, float* __restrict__ w, __nv_bfloat16* __
 #pragma unroll
   for (int j = 0; j < VPT; ++j) {
     int e = lane + 32 * j;
-    sel[j] = e < n ? (bias ? s[j] + bias[e] : s[j]) : -INFINITY;
+    sel[j] = e < n ? (a.bias ? s[j] + a.bias[e] : s[j]) : -INFINITY;
   }
-  if (n_groups > 1) group_mask<VPT>(sel, n, n_groups, topk_groups, B200MOE_F32, lane);
+  if (a.n_groups > 1) group_mask<VPT>(sel, n, a.n_groups, a.topk_groups, B200MOE_F32, lane);
   float rv;
   int ri;
   warp_topk<VPT>(sel, n, k, lane, rv, ri);
@@ -198,36 +202,56 @@ route_kernel(int32_t* __restrict__ ids, float* __restrict__ w, __nv_bfloat16* __
     if ((ri >> 5) == j) wv = cand;
   }
   if (lane >= k) wv = 0.f;
-  if (renorm) {
+  if (a.renorm) {
     float sum = wv;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
     wv = wv / sum;
   }
-  wv = wv * scale;
+  wv = wv * a.scale;
   if (lane < k) {
-    ids[row * k + lane] = ri;
-    w[row * k + lane] = wv;
-    if (w_bf16) w_bf16[row * k + lane] = __float2bfloat16_rn(wv);
+    a.ids[row * k + lane] = ri;
+    a.w[row * k + lane] = wv;
+    if (a.w_bf16) a.w_bf16[row * k + lane] = __float2bfloat16_rn(wv);
   }
+}
+
+template <int VPT>
+__global__ void __launch_bounds__(kWarpsPerBlock * 32)
+route_kernel(const float* __restrict__ logits, int64_t T, int n, const RouteArgs a) {
+  pdl_begin();
+  const int lane = threadIdx.x & 31;
+  const int64_t row = (int64_t)blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
+  if (row >= T) return;
+  float s[VPT];
+#pragma unroll
+  for (int j = 0; j < VPT; ++j) {
+    int e = lane + 32 * j;
+    s[j] = e < n ? logits[row * n + e] : -INFINITY;
+  }
+  route_row<VPT>(s, a, row, n, lane);
 }
 
 // ---- router GEMM ---------------------------------------------------------------------------------
 // logits[t,e] = sum_h x[t,h] * wr[e,h]; bf16 operands, fp32 accumulation on the warp-level tensor path
 // (mma.sync m16n8k16).  It is ~0.5 % of the layer's FLOPs and bound by the copies of x and wr on their way to shared
-// memory, so what counts is how many of them are in flight: a block owns 64 tokens x 128 experts (x is read once up to
-// 128 experts), four stages of 64 K columns, and when that leaves SMs without a block the K range is split over the
-// blocks of a cluster, which add their tiles up through distributed shared memory, in rank order (the result does not
-// depend on timing).  Measured against 32 x 64 tiles that walk all of K (64 tokens of the DeepSeek shape were 8 blocks
-// with 112 dependent steps each): 42 -> 15 us there, 57 -> 43 us at 2048 tokens,
-// 34 -> 25 us for 8192 tokens of the Qwen3 shape.
-constexpr int RG_BM = 64, RG_BN = 128, RG_BK = 64, RG_LD = RG_BK + 8, RG_STAGES = 4;  // +8 bf16: conflict-free ldmatrix
-constexpr int RG_THREADS = 256;
-constexpr int RG_STAGE_ELEMS = (RG_BM + RG_BN) * RG_LD;
-constexpr size_t RG_SMEM_BYTES = (size_t)RG_STAGES * RG_STAGE_ELEMS * sizeof(__nv_bfloat16);
-constexpr int RG_CLD = RG_BN + 4;  // fp32 tile on its way between the blocks of a cluster
-static_assert((size_t)RG_BM * RG_CLD * sizeof(float) <= RG_SMEM_BYTES, "the fp32 tile reuses the stages");
-constexpr int RG_MAX_SPLIT = 8;  // portable cluster size
+// memory and by the chain of MMAs over K.  That chain is never cut: a logit is the same number whatever the tile and the
+// batch size (K in order), so that a token's experts do not depend on them - cutting it moves logits by 1e-6, which gave
+// one token in a few thousand other experts.  So the batch decides the tile instead, the largest that gives most SMs a
+// block; stages are four or eight 64-column chunks deep.  Against 32 x 64 tiles and three stages for every batch: DeepSeek
+// shape 64 tokens 42 -> 25 us (8 blocks became 64), 2048 tokens 57 -> 52, Qwen3 shape 8192 tokens 34 -> 27.
+constexpr int RG_BK = 64, RG_LD = RG_BK + 8;  // +8 bf16: conflict-free ldmatrix
+template <int BM_, int BN_, int WM_, int WN_, int STAGES_>
+struct RgTile {
+  static constexpr int BM = BM_, BN = BN_, WM = WM_, WN = WN_, STAGES = STAGES_;  // WM x WN warps
+  static constexpr int THREADS = 32 * WM * WN, MT = BM / WM / 16, NT = BN / WN / 8;
+  static constexpr int STAGE_ELEMS = (BM + BN) * RG_LD;
+  static constexpr size_t SMEM = (size_t)STAGES * STAGE_ELEMS * sizeof(__nv_bfloat16);
+  static_assert(BM == WM * MT * 16 && BN == WN * NT * 8 && (NT == 1 || NT % 2 == 0) && (BM + BN) * 8 % THREADS == 0, "");
+};
+using RgLarge = RgTile<64, 128, 2, 4, 4>;
+using RgMedium = RgTile<32, 64, 2, 2, 4>;
+using RgSmall = RgTile<16, 16, 1, 2, 8>;
 
 __device__ __forceinline__ void mma_bf16_16816(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
   asm volatile(
@@ -240,6 +264,11 @@ __device__ __forceinline__ void ldmatrix_x4(uint32_t (&r)[4], const void* p) {
                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
                : "r"((uint32_t)__cvta_generic_to_shared(p)));
 }
+__device__ __forceinline__ void ldmatrix_x2(uint32_t& r0, uint32_t& r1, const void* p) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x2.shared.b16 {%0,%1}, [%2];"
+               : "=r"(r0), "=r"(r1)
+               : "r"((uint32_t)__cvta_generic_to_shared(p)));
+}
 
 // 16-byte asynchronous copy global -> shared; bytes = 0 writes zeros (rows / columns past the end)
 __device__ __forceinline__ void cp_async16(void* smem_dst, const void* gsrc, int bytes) {
@@ -248,35 +277,34 @@ __device__ __forceinline__ void cp_async16(void* smem_dst, const void* gsrc, int
                : "memory");
 }
 
-// grid (ceil(T / 64), splits, ceil(E / 128)), clusters of (1, splits, 1)
-__global__ void __launch_bounds__(RG_THREADS)
+// grid (ceil(T / BM), ceil(E / BN))
+template <class C>
+__global__ void __launch_bounds__(C::THREADS)
 router_gemm_kernel(float* __restrict__ logits, const __nv_bfloat16* __restrict__ x,
                    const __nv_bfloat16* __restrict__ wr, int64_t T, int64_t H, int64_t E) {
   pdl_begin();
   extern __shared__ __align__(16) uint8_t rg_smem[];
   __nv_bfloat16* const stages = reinterpret_cast<__nv_bfloat16*>(rg_smem);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int wm = warp & 1, wn = warp >> 1;  // the warp's 32 rows and 32 columns of the 64 x 128 tile
-  const int splits = gridDim.y, rank = blockIdx.y;
-  const int64_t t0 = (int64_t)blockIdx.x * RG_BM, e0 = (int64_t)blockIdx.z * RG_BN;
+  const int row_w = (warp % C::WM) * (C::MT * 16), col_w = (warp / C::WM) * (C::NT * 8);  // the warp's part of the tile
+  const int64_t t0 = (int64_t)blockIdx.x * C::BM, e0 = (int64_t)blockIdx.y * C::BN;
   const int nk = (int)((H + RG_BK - 1) / RG_BK);
-  const int k_begin = (int)((int64_t)nk * rank / splits), k_end = (int)((int64_t)nk * (rank + 1) / splits);
-  float acc[2][4][4];
+  float acc[C::MT][C::NT][4];
 #pragma unroll
-  for (int m = 0; m < 2; ++m)
+  for (int m = 0; m < C::MT; ++m)
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+    for (int i = 0; i < C::NT; ++i)
 #pragma unroll
       for (int j = 0; j < 4; ++j) acc[m][i][j] = 0.f;
   auto load_stage = [&](int kt) {
-    __nv_bfloat16* const st = stages + (size_t)((kt - k_begin) % RG_STAGES) * RG_STAGE_ELEMS;
+    __nv_bfloat16* const st = stages + (size_t)(kt % C::STAGES) * C::STAGE_ELEMS;
     const int64_t k0 = (int64_t)kt * RG_BK;
 #pragma unroll
-    for (int i = 0; i < (RG_BM + RG_BN) * 8 / RG_THREADS; ++i) {  // rows of x, then rows of wr; 8 chunks of 16 B each
-      const int c = tid + i * RG_THREADS;
+    for (int i = 0; i < (C::BM + C::BN) * 8 / C::THREADS; ++i) {  // rows of x, then rows of wr; 8 chunks of 16 B each
+      const int c = tid + i * C::THREADS;
       const int r = c >> 3, cc = (c & 7) * 8;
-      const bool is_x = r < RG_BM;
-      const int64_t row = is_x ? t0 + r : e0 + r - RG_BM;
+      const bool is_x = r < C::BM;
+      const int64_t row = is_x ? t0 + r : e0 + r - C::BM;
       const bool on = k0 + cc < H && row < (is_x ? T : E);
       const __nv_bfloat16* src = (is_x ? x : wr) + (on ? row * H + k0 + cc : 0);
       cp_async16(st + r * RG_LD + cc, src, on ? 16 : 0);
@@ -285,78 +313,50 @@ router_gemm_kernel(float* __restrict__ logits, const __nv_bfloat16* __restrict__
   // one commit group per chunk, empty where there is no chunk left, so that "all but the newest groups are complete"
   // always means "chunk kt has landed"
 #pragma unroll
-  for (int s = 0; s < RG_STAGES - 1; ++s) {
-    if (k_begin + s < k_end) load_stage(k_begin + s);
+  for (int s = 0; s < C::STAGES - 1; ++s) {
+    if (s < nk) load_stage(s);
     asm volatile("cp.async.commit_group;" ::: "memory");
   }
-  for (int kt = k_begin; kt < k_end; ++kt) {
-    asm volatile("cp.async.wait_group %0;" ::"n"(RG_STAGES - 2) : "memory");
+  for (int kt = 0; kt < nk; ++kt) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(C::STAGES - 2) : "memory");
     __syncthreads();  // chunk kt is there for everyone, and everyone is done with the stage that is filled next
-    if (kt + RG_STAGES - 1 < k_end) load_stage(kt + RG_STAGES - 1);
+    if (kt + C::STAGES - 1 < nk) load_stage(kt + C::STAGES - 1);
     asm volatile("cp.async.commit_group;" ::: "memory");
-    const __nv_bfloat16* sA = stages + (size_t)((kt - k_begin) % RG_STAGES) * RG_STAGE_ELEMS;
-    const __nv_bfloat16* sB = sA + RG_BM * RG_LD;
+    const __nv_bfloat16* sA = stages + (size_t)(kt % C::STAGES) * C::STAGE_ELEMS;
+    const __nv_bfloat16* sB = sA + C::BM * RG_LD;
 #pragma unroll
     for (int kk = 0; kk < RG_BK; kk += 16) {
-      uint32_t a[2][4], b[2][4];
+      uint32_t a[C::MT][4], b[C::NT][2];
 #pragma unroll
-      for (int m = 0; m < 2; ++m)  // rows 0-7 / 8-15 at k, then the same at k + 8
-        ldmatrix_x4(a[m], sA + (wm * 32 + m * 16 + (lane & 15)) * RG_LD + kk + (lane >> 4) * 8);
+      for (int m = 0; m < C::MT; ++m)  // rows 0-7 / 8-15 at k, then the same at k + 8
+        ldmatrix_x4(a[m], sA + (row_w + m * 16 + (lane & 15)) * RG_LD + kk + (lane >> 4) * 8);
+      if (C::NT == 1) {
+        ldmatrix_x2(b[0][0], b[0][1], sB + (col_w + (lane & 7)) * RG_LD + kk + ((lane >> 3) & 1) * 8);
+      } else {
 #pragma unroll
-      for (int p = 0; p < 2; ++p)  // columns 0-7 at k, k + 8, then columns 8-15
-        ldmatrix_x4(b[p], sB + (wn * 32 + p * 16 + (lane & 7) + ((lane >> 4) << 3)) * RG_LD + kk + ((lane >> 3) & 1) * 8);
+        for (int p = 0; p < C::NT / 2; ++p) {  // columns 0-7 at k, k + 8, then columns 8-15
+          uint32_t r[4];
+          ldmatrix_x4(r, sB + (col_w + p * 16 + (lane & 7) + ((lane >> 4) << 3)) * RG_LD + kk + ((lane >> 3) & 1) * 8);
+          b[2 * p][0] = r[0], b[2 * p][1] = r[1];
+          b[(2 * p + 1) % C::NT][0] = r[2], b[(2 * p + 1) % C::NT][1] = r[3];
+        }
+      }
 #pragma unroll
-      for (int m = 0; m < 2; ++m)
+      for (int m = 0; m < C::MT; ++m)
 #pragma unroll
-        for (int nb = 0; nb < 4; ++nb) mma_bf16_16816(acc[m][nb], a[m], b[nb >> 1][(nb & 1) * 2], b[nb >> 1][(nb & 1) * 2 + 1]);
+        for (int nb = 0; nb < C::NT; ++nb) mma_bf16_16816(acc[m][nb], a[m], b[nb][0], b[nb][1]);
     }
   }
   const int g = lane >> 2, tq = lane & 3;
-  if (splits == 1) {
 #pragma unroll
-    for (int m = 0; m < 2; ++m)
+  for (int m = 0; m < C::MT; ++m)
 #pragma unroll
-      for (int nb = 0; nb < 4; ++nb)
+    for (int nb = 0; nb < C::NT; ++nb)
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const int64_t r = t0 + wm * 32 + m * 16 + g + (i >> 1) * 8, c = e0 + wn * 32 + nb * 8 + tq * 2 + (i & 1);
-          if (r < T && c < E) logits[r * E + c] = acc[m][nb][i];
-        }
-    return;
-  }
-  asm volatile("cp.async.wait_group 0;" ::: "memory");
-  __syncthreads();  // the stages are free: the tile goes there
-  float* const tile = reinterpret_cast<float*>(rg_smem);
-#pragma unroll
-  for (int m = 0; m < 2; ++m)
-#pragma unroll
-    for (int nb = 0; nb < 4; ++nb)
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-        tile[(wm * 32 + m * 16 + g + (i >> 1) * 8) * RG_CLD + wn * 32 + nb * 8 + tq * 2 + (i & 1)] = acc[m][nb][i];
-  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-  // every block sums and stores its share of the tile's rows
-  const uint32_t tile_addr = (uint32_t)__cvta_generic_to_shared(tile);
-  const int rows = RG_BM / splits;
-  for (int i = tid; i < rows * (RG_BN / 4); i += RG_THREADS) {
-    const int r = rank * rows + i / (RG_BN / 4), c = (i % (RG_BN / 4)) * 4;
-    float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
-    for (int p = 0; p < splits; ++p) {
-      uint32_t addr;
-      float4 v;
-      asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(addr) : "r"(tile_addr + (uint32_t)(r * RG_CLD + c) * 4u), "r"(p));
-      asm volatile("ld.shared::cluster.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
-      sum.x += v.x, sum.y += v.y, sum.z += v.z, sum.w += v.w;
-    }
-    if (t0 + r < T) {
-      float* dst = logits + (t0 + r) * E + e0 + c;
-      const float s4[4] = {sum.x, sum.y, sum.z, sum.w};
-#pragma unroll
-      for (int u = 0; u < 4; ++u)
-        if (e0 + c + u < E) dst[u] = s4[u];
-    }
-  }
-  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");  // no block leaves while its tile is read
+      for (int i = 0; i < 4; ++i) {
+        const int64_t r = t0 + row_w + m * 16 + g + (i >> 1) * 8, c = e0 + col_w + nb * 8 + tq * 2 + (i & 1);
+        if (r < T && c < E) logits[r * E + c] = acc[m][nb][i];
+      }
 }
 
 // Small-T variant (decode): one block per expert row; its 4 warps split H (16-byte loads) and dot the slice with up
@@ -408,12 +408,14 @@ constexpr int RS_TOK = 4, RS_WARPS = 8;
 // op is a read of x.  A block owns RS_TOK tokens and its 8 warps split H between them (interleaved 256-column
 // slices, 16-byte loads of x and of the L2-resident router weights), so that decode-size batches still fill more
 // than a handful of SMs; the per-warp partial sums meet in shared memory and are added in warp order, so the
-// result does not depend on timing.
-template <int EP>
+// result does not depend on timing.  With ROUTE the block goes on to route its tokens, one warp each, from the logits it
+// has just formed: one launch less in front of the experts (Mixtral shape, 32 tokens: 6.6 + 3.5 us as two kernels).
+template <int EP, bool ROUTE>
 __global__ void __launch_bounds__(RS_WARPS * 32)
 router_small_e_kernel(float* __restrict__ logits, const __nv_bfloat16* __restrict__ x,
-                       const __nv_bfloat16* __restrict__ wr, int64_t T, int64_t H, int E) {
+                       const __nv_bfloat16* __restrict__ wr, int64_t T, int64_t H, int E, const RouteArgs ra) {
   pdl_begin();
+  __shared__ float sums[RS_TOK][EP];
   __shared__ float part[RS_WARPS][RS_TOK][EP];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int64_t t0 = (int64_t)blockIdx.x * RS_TOK;
@@ -468,7 +470,30 @@ router_small_e_kernel(float* __restrict__ logits, const __nv_bfloat16* __restric
 #pragma unroll
     for (int w = 0; w < RS_WARPS; ++w) v += part[w][i][e];
     if (t0 + i < T && e < E) logits[(t0 + i) * E + e] = v;
+    if (ROUTE) sums[i][e] = v;
   }
+  if (ROUTE) {
+    __syncthreads();
+    if (warp < RS_TOK && t0 + warp < T) {
+      float s[1] = {lane < EP ? sums[warp][lane] : 0.f};  // (elements >= E are masked by route_row)
+      route_row<1>(s, ra, t0 + warp, E, lane);
+    }
+  }
+}
+
+template <class C>
+int launch_router_gemm(float* logits, const __nv_bfloat16* x, const __nv_bfloat16* wr, int64_t T, int64_t H, int64_t E,
+                       cudaStream_t st) {
+  constexpr int kMaxDevices = 64;
+  static bool attr_done[kMaxDevices] = {};
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return B200MOE_EDRIVER;
+  if (!attr_done[dev]) {  // per-device attribute
+    cudaFuncSetAttribute(router_gemm_kernel<C>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::SMEM);
+    attr_done[dev] = true;
+  }
+  return moe_launch(router_gemm_kernel<C>, dim3((unsigned)((T + C::BM - 1) / C::BM), (unsigned)((E + C::BN - 1) / C::BN)),
+                    C::THREADS, C::SMEM, st, logits, x, wr, T, H, E);
 }
 
 template <typename F>
@@ -513,9 +538,9 @@ extern "C" int b200moe_topk(void* values, int32_t* indices, const void* x, int d
   return launch_topk(values, indices, x, dtype, batch, n, 1, 1, k, stream);
 }
 
-extern "C" int b200moe_route(int32_t* ids, float* w, void* w_bf16, const float* logits,
-                             const float* logit_bias, const float* bias, int64_t T, int64_t E, int64_t k, int score_func, int64_t n_groups,
-                             int64_t topk_groups, int renorm, float scale, void* stream) {
+namespace {
+int check_route(const void* ids, const void* w, const void* logits, int64_t T, int64_t E, int64_t k, int score_func,
+                int64_t n_groups, int64_t topk_groups) {
   MOE_CHECK_ARG(ids && w && logits && T >= 0 && E > 0 && k > 0);
   MOE_CHECK_ARG(score_func == B200MOE_SCORE_SOFTMAX || score_func == B200MOE_SCORE_SIGMOID);
   MOE_CHECK_SHAPE(E <= 1024 && k <= 32 && k <= E);
@@ -523,13 +548,50 @@ extern "C" int b200moe_route(int32_t* ids, float* w, void* w_bf16, const float* 
     MOE_CHECK_SHAPE(n_groups <= 32 && E % n_groups == 0 && topk_groups >= 1 && topk_groups <= n_groups);
     MOE_CHECK_SHAPE(k <= topk_groups * (E / n_groups));
   }
+  return B200MOE_OK;
+}
+RouteArgs route_args(int32_t* ids, float* w, void* w_bf16, const float* logit_bias, const float* bias, int64_t k,
+                     int score_func, int64_t n_groups, int64_t topk_groups, int renorm, float scale) {
+  return RouteArgs{ids, w, reinterpret_cast<__nv_bfloat16*>(w_bf16), logit_bias, bias, (int)k, score_func,
+                   (int)(n_groups > 1 ? n_groups : 1), (int)topk_groups, renorm, scale};
+}
+}  // namespace
+
+extern "C" int b200moe_route(int32_t* ids, float* w, void* w_bf16, const float* logits,
+                             const float* logit_bias, const float* bias, int64_t T, int64_t E, int64_t k, int score_func, int64_t n_groups,
+                             int64_t topk_groups, int renorm, float scale, void* stream) {
+  const int rc = check_route(ids, w, logits, T, E, k, score_func, n_groups, topk_groups);
+  if (rc) return rc;
   if (T == 0) return B200MOE_OK;
+  const RouteArgs a = route_args(ids, w, w_bf16, logit_bias, bias, k, score_func, n_groups, topk_groups, renorm, scale);
   dim3 grid((unsigned)((T + kWarpsPerBlock - 1) / kWarpsPerBlock));
   return dispatch_vpt(E, [&](auto vpt) {
-    return moe_launch(route_kernel<decltype(vpt)::value>, grid, kWarpsPerBlock * 32, 0, (cudaStream_t)stream, ids, w,
-                      reinterpret_cast<__nv_bfloat16*>(w_bf16), logits, logit_bias, bias, T, (int)E, (int)k, score_func,
-                      (int)(n_groups > 1 ? n_groups : 1), (int)topk_groups, renorm, scale);
+    return moe_launch(route_kernel<decltype(vpt)::value>, grid, kWarpsPerBlock * 32, 0, (cudaStream_t)stream, logits, T,
+                      (int)E, a);
   });
+}
+
+extern "C" int b200moe_router_route(float* logits, int32_t* ids, float* w, void* w_bf16, const void* x, const void* wr,
+                                    const float* logit_bias, const float* bias, int64_t T, int64_t H, int64_t E, int64_t k,
+                                    int score_func, int64_t n_groups, int64_t topk_groups, int renorm, float scale,
+                                    void* stream) {
+  int rc = check_route(ids, w, logits, T, E, k, score_func, n_groups, topk_groups);
+  if (rc) return rc;
+  // One kernel where the few-experts variant forms the logits, which holds all of a token's in one block; the other
+  // variants, and the small batches that spread every expert row over a block, route in a second one.
+  if (E > 16 || T <= 2 * RV_MAXT) {
+    rc = b200moe_router_logits(logits, x, wr, T, H, E, stream);
+    if (rc) return rc;
+    return b200moe_route(ids, w, w_bf16, logits, logit_bias, bias, T, E, k, score_func, n_groups, topk_groups, renorm, scale,
+                         stream);
+  }
+  MOE_CHECK_ARG(x && wr && H > 0);
+  MOE_CHECK_SHAPE(H % 8 == 0);
+  if (!moe_aligned16(x) || !moe_aligned16(wr)) return B200MOE_EALIGN;
+  const RouteArgs a = route_args(ids, w, w_bf16, logit_bias, bias, k, score_func, n_groups, topk_groups, renorm, scale);
+  return moe_launch(E <= 8 ? router_small_e_kernel<8, true> : router_small_e_kernel<16, true>,
+                    dim3((unsigned)((T + RS_TOK - 1) / RS_TOK)), RS_WARPS * 32, 0, (cudaStream_t)stream, logits,
+                    reinterpret_cast<const __nv_bfloat16*>(x), reinterpret_cast<const __nv_bfloat16*>(wr), T, H, (int)E, a);
 }
 
 extern "C" int b200moe_router_logits(float* logits, const void* x, const void* wr, int64_t T, int64_t H,
@@ -544,21 +606,14 @@ extern "C" int b200moe_router_logits(float* logits, const void* x, const void* w
     return moe_launch(router_gemv_kernel, dim3((unsigned)E, (unsigned)((T + RV_MAXT - 1) / RV_MAXT)), 128, 0,
                       (cudaStream_t)stream, logits, xb, wb, T, H, E);
   } else if (E <= 16) {
-    return moe_launch(E <= 8 ? router_small_e_kernel<8> : router_small_e_kernel<16>, dim3((unsigned)((T + RS_TOK - 1) / RS_TOK)),
-                      RS_WARPS * 32, 0, (cudaStream_t)stream, logits, xb, wb, T, H, (int)E);
+    return moe_launch(E <= 8 ? router_small_e_kernel<8, false> : router_small_e_kernel<16, false>, dim3((unsigned)((T + RS_TOK - 1) / RS_TOK)),
+                      RS_WARPS * 32, 0, (cudaStream_t)stream, logits, xb, wb, T, H, (int)E, RouteArgs{});
   } else {
-    constexpr int kMaxDevices = 64;
-    static bool attr_done[kMaxDevices] = {};
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return B200MOE_EDRIVER;
-    if (!attr_done[dev]) {  // per-device attribute
-      cudaFuncSetAttribute(router_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)RG_SMEM_BYTES);
-      attr_done[dev] = true;
-    }
-    const int64_t mt = (T + RG_BM - 1) / RG_BM, nt = (E + RG_BN - 1) / RG_BN;
-    int splits = 1;  // as many as there are SMs for, with at least 256 columns of K each
-    while (splits < RG_MAX_SPLIT && mt * nt * splits * 2 <= moe_device_sm_count() && H / (splits * 2) >= 4 * RG_BK) splits *= 2;
-    return moe_launch_cluster(splits, router_gemm_kernel, dim3((unsigned)mt, (unsigned)splits, (unsigned)nt), RG_THREADS,
-                              RG_SMEM_BYTES, (cudaStream_t)stream, logits, xb, wb, T, H, E);
+    // the larger tile where it still gives most SMs a block
+    auto blocks = [&](int bm, int bn) { return ((T + bm - 1) / bm) * ((E + bn - 1) / bn); };
+    const int64_t enough = moe_device_sm_count() * 4 / 5;
+    if (blocks(RgLarge::BM, RgLarge::BN) >= enough) return launch_router_gemm<RgLarge>(logits, xb, wb, T, H, E, (cudaStream_t)stream);
+    if (blocks(RgMedium::BM, RgMedium::BN) >= enough) return launch_router_gemm<RgMedium>(logits, xb, wb, T, H, E, (cudaStream_t)stream);
+    return launch_router_gemm<RgSmall>(logits, xb, wb, T, H, E, (cudaStream_t)stream);
   }
 }

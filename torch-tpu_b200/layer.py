@@ -59,9 +59,9 @@ class FusedMoE:
     def route(self, x):
         T = x.shape[0]
         c = self.cfg
-        logits = ops.router_logits(x, self.router_w, out=self.logits[:T])
-        return ops.route(logits, c.top_k, c.score_func, self.bias, c.n_groups, c.topk_groups, c.renorm,
-                         c.routed_scale, ids=self.ids[:T], w=self.topk_w[:T], logit_bias=self.logit_bias)
+        return ops.router_route(x, self.router_w, c.top_k, c.score_func, self.bias, c.n_groups, c.topk_groups, c.renorm,
+                                c.routed_scale, logits=self.logits[:T], ids=self.ids[:T], w=self.topk_w[:T],
+                                logit_bias=self.logit_bias)
 
     def forward(self, x, out=None):
         """x bf16 [T,H] on the device -> bf16 [T,H] (a view of an internal buffer unless ``out`` is given)."""

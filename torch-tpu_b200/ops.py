@@ -75,6 +75,26 @@ def route(logits, k, score_func="softmax", bias=None, n_groups=1, topk_groups=1,
     return ids, w
 
 
+def router_route(x, wr, k, score_func="softmax", bias=None, n_groups=1, topk_groups=1, renorm=True, scale=1.0,
+                 logits=None, ids=None, w=None, logit_bias=None):
+    """router_logits and route in one call (one kernel for at most 16 experts and more than 16 tokens).  Returns (ids int32 [T,k], w fp32 [T,k])."""
+    _chk(x, "x", torch.bfloat16)
+    _chk(wr, "wr", torch.bfloat16)
+    T, H = x.shape
+    E = wr.shape[0]
+    if logits is None:
+        logits = torch.empty(T, E, dtype=torch.float32, device=x.device)
+    if ids is None:
+        ids = torch.empty(T, k, dtype=torch.int32, device=x.device)
+    if w is None:
+        w = torch.empty(T, k, dtype=torch.float32, device=x.device)
+    sf = L.SCORE_SOFTMAX if score_func == "softmax" else L.SCORE_SIGMOID
+    L.check(L.lib().b200moe_router_route(_ptr(logits), _ptr(ids), _ptr(w), _ptr(None), _ptr(x), _ptr(wr), _ptr(logit_bias),
+                                         _ptr(bias), T, H, E, k, sf, n_groups, topk_groups, int(renorm), float(scale),
+                                         _stream()), "b200moe_router_route")
+    return ids, w
+
+
 def permute(ids, num_experts, status=None):
     """Stable sort of the (token,slot) pairs by expert.  Returns (sorted_pair int32 [P], expert_offsets int32 [E+1])."""
     _chk(ids, "ids", torch.int32)
