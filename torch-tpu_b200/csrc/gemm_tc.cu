@@ -876,7 +876,7 @@ int launch_tc(const MoeGemmArgs& g, cudaStream_t st) {
   const int grid = (int)((a.part ? max_tiles * kMaxParts : max_tiles) < sms ? (a.part ? max_tiles * kMaxParts : max_tiles) : sms);
   if (grid > kMaxSplitCtas) a.part = nullptr;  // the slots are laid out for that many
   a.lists_ready = g.lists_ready;
-  return moe_launch(moe_gemm_tc_kernel<MODE>, grid, TC_THREADS, TC_SMEM_BYTES, st, tmA, tmAs, tmB0, tmB1, a);
+  return moe_launch_as(g.P <= kOverlapMaxRows, 1, moe_gemm_tc_kernel<MODE>, grid, TC_THREADS, TC_SMEM_BYTES, st, tmA, tmAs, tmB0, tmB1, a);
 }
 
 }  // namespace

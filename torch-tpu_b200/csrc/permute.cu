@@ -419,7 +419,7 @@ int moe_permute_impl(int32_t* sorted_pair, int32_t* expert_offsets, const int32_
   MOE_CHECK_ARG(scratch);
   const int nchunks = (int)((P + kChunk - 1) / kChunk);
   if (nchunks <= kMaxCluster)
-    return moe_launch_cluster(nchunks, permute_cluster_kernel, dim3(1, nchunks), kChunk, smem, st, ids, P, (int)E,
+    return moe_launch_as(true, nchunks, permute_cluster_kernel, dim3(1, nchunks), kChunk, smem, st, ids, P, (int)E,
                               expert_offsets, sorted_pair, status, mtiles, num_mtiles, max_mtiles, pos_of, split_cnt);
   int rc = moe_launch(permute_hist_kernel, nchunks, kChunk, smem, st, ids, P, (int)E, scratch, status);
   if (!rc) rc = moe_launch(permute_scan_kernel, 1, kChunk, 0, st, scratch, nchunks, (int)E, expert_offsets, mtiles, num_mtiles,
