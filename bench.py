@@ -234,22 +234,24 @@ def median(v):
 
 def launches_per_step(wl, T, world=1, ep="nccl"):
     P = T * wl["k"]
+    route = 1 if wl["E"] <= 16 and T > 16 else 2        # router and selection (one kernel for few experts)
+    sort = lambda pairs: 1 if pairs <= 8192 else 3
     if world > 1 and ep == "p2p":
         # router, route, permute | counts exchange, plan, dispatch, barrier | scales, tiles, 2 GEMMs, barrier | combine
-        n = 2 + (1 if P <= 1024 else 3) + 4 + 5 + 1
+        n = route + sort(P) + 4 + 5 + 1
         if wl.get("shared"):
-            n += (1 if T <= 1024 else 3) + 1 + 1 + 2
+            n += sort(T) + 1 + 2
         return n
     if world > 1:
         # router, route, permute, pack | unpack ids, permute (received rows), unpack rows, tiles, 2 GEMMs | invert, combine
-        n = 2 + (1 if P <= 1024 else 3) + 1 + 1 + 3 + 1 + 1 + 2 + 2
+        n = route + sort(P) + 1 + 1 + 3 + 1 + 1 + 2 + 2
         if wl.get("shared"):
-            n += (1 if T <= 1024 else 3) + 1 + 1 + 2      # permute (identity ids), tiles, quant, 2 GEMMs
+            n += sort(T) + 1 + 2                          # permute (identity ids, tiles with it), quant, 2 GEMMs
         return n
-    # router, route, permute (+ tiles: one kernel up to 1024 pairs, else 3 + 1), quant, 2 GEMMs, combine
-    n = 2 + (1 if P <= 1024 else 4) + 1 + 2 + 1
+    # router, route, permute (tiles with it), quant, 2 GEMMs, combine
+    n = route + sort(P) + 1 + 2 + 1
     if wl.get("shared"):
-        n += 2 + 1 + 2                                  # identity offsets + tiles, quant, 2 GEMMs
+        n += 1 + 2                                        # quant (lists with it), 2 GEMMs
     return n
 
 
