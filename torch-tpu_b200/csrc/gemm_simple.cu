@@ -237,7 +237,7 @@ __global__ void __launch_bounds__(256) identity_lists_kernel(MoeIdentityLists li
 
 // out[t,:] = bf16( sum_j w[t,j]*y[t,j,:] (+ add[t,:]) ); one thread per 8 columns (16-byte accesses).  The rows of four
 // slots are requested before the first is used, the sum is formed in slot order: taken slot by slot a thread waits for
-// one memory round trip per slot (Qwen3 shape, 8192 tokens x 8 slots: 68 us for 300 MB).
+// one memory round trip per slot (Qwen3 shape, 8192 tokens x 8 slots, 300 MB: 68 -> 54 us).
 constexpr int CB_SLOTS = 4;
 __global__ void __launch_bounds__(256)
 combine_kernel(__nv_bfloat16* __restrict__ out, const __nv_bfloat16* __restrict__ y, const void* __restrict__ w,
