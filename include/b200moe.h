@@ -107,7 +107,7 @@ int b200moe_route(int32_t* ids, float* w, void* w_bf16, const float* logits, con
                   const float* bias, int64_t T, int64_t E, int64_t k, int score_func, int64_t n_groups,
                   int64_t topk_groups, int renorm, float scale, void* stream);
 
-/* b200moe_router_logits and b200moe_route in one call (with at most 16 experts and more than 16 tokens in one kernel): logits, ids and w are all
+/* b200moe_router_logits and b200moe_route in one call (one kernel for a few hundred tokens and at most 16 experts): logits, ids and w are all
  * written.  Same limits as the two. */
 int b200moe_router_route(float* logits, int32_t* ids, float* w, void* w_bf16, const void* x, const void* wr,
                          const float* logit_bias, const float* bias, int64_t T, int64_t H, int64_t E, int64_t k,

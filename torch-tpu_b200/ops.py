@@ -77,7 +77,7 @@ def route(logits, k, score_func="softmax", bias=None, n_groups=1, topk_groups=1,
 
 def router_route(x, wr, k, score_func="softmax", bias=None, n_groups=1, topk_groups=1, renorm=True, scale=1.0,
                  logits=None, ids=None, w=None, logit_bias=None):
-    """router_logits and route in one call (one kernel for at most 16 experts and more than 16 tokens).  Returns (ids int32 [T,k], w fp32 [T,k])."""
+    """router_logits and route in one call (one kernel for a few hundred tokens and at most 16 experts).  Returns (ids int32 [T,k], w fp32 [T,k])."""
     _chk(x, "x", torch.bfloat16)
     _chk(wr, "wr", torch.bfloat16)
     T, H = x.shape
