@@ -235,7 +235,9 @@ moe_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer of the weights (one thread)
     // Two producers, this one for B and warp 3's for A, each on its own clock.  Weights are nobody's output: where the
-    // work list is ready they are requested before the kernel in front of this one has finished.
+    // work list is ready the first TC_STAGES blocks are requested before the kernel in front of this one has finished.
+    // The waits for a stage to come free begin after it has: their limit covers this kernel's own progress, however long
+    // the other one takes.
     if (lane == 0) {
       bool ok = true;
       // the m-tile list entry of the NEXT work item is requested while this one's loads are issued: when the weights
@@ -247,6 +249,7 @@ moe_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
         nx_e = a.mtiles[2 * nx.mt];
       }
       uint32_t s = 0, ph = 1;
+      int ahead = TC_STAGES;  // stages that are free from the start
       for (int t = blockIdx.x; t < total_tiles && ok; t += gridDim.x) {
         const int KB = nx.KB;
         // coordinates of the two boxes of the first K block, and their step per K block
@@ -259,6 +262,7 @@ moe_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
         int row = n0, col = c0;
         for (int kb = 0; kb < KB; ++kb) {
           const uint32_t full = smem_u32(&sh->full[0]) + s * 8, sb = smem_base + TC_A_BYTES + s * TC_STAGE_BYTES;
+          if (ahead-- == 0) pdl_wait();
           if (!mbar_wait(smem_u32(&sh->empty[0]) + s * 8, ph, abort_flag)) {
             ok = false;
             break;
@@ -291,6 +295,7 @@ moe_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
           n_it += (uint32_t)((int)((int64_t)KB_all * (ks + 1) / a.KS) - (int)((int64_t)KB_all * ks / a.KS));
         }
       }
+      pdl_wait();  // no operand is complete before that, and the waits' limit is for this kernel alone
       for (uint32_t it = 0; it < n_it; ++it) {
         const uint32_t s = it % TC_STAGES, buf = it & 1;
         if (!mbar_wait(smem_u32(&sh->full[s]), (it / TC_STAGES) & 1, abort_flag)) break;
