@@ -24,6 +24,37 @@ def _raw_weights(E, H, I, seed):
     return (*w, *s)
 
 
+@pytest.mark.parametrize("tokens", [2048, 4096])
+def test_capped_grid_leaves_sms_to_another_stream(m, tokens):
+    """max_ctas = n: the other SMs stay free for another stream's kernels for as long as the call runs.  The gate/up GEMM
+    of one expert on 98 SMs takes hundreds of microseconds and is two thirds of the call; a permutation on another
+    stream takes tens.  If the down GEMM's CTAs, or the kernels behind them, already sit on the free SMs and wait, the
+    permutation cannot end before the gate/up GEMM does."""
+    H, I, E = 4096, 14336, 1
+    w = _raw_weights(E, H, I, 5)
+    x = torch.randn(tokens, H, device=DEV).to(torch.bfloat16)
+    ids = torch.zeros(tokens, 1, dtype=torch.int32, device=DEV)
+    out = torch.empty(tokens, 1, H, dtype=torch.bfloat16, device=DEV)
+    other = torch.randint(0, 64, (1024, 4), dtype=torch.int32, device=DEV)
+    d = m.ops.make_desc(tokens, H, I, E, 1, max_ctas=98)
+    ws = torch.empty(m.ops.experts_workspace_bytes(d) + 256, dtype=torch.uint8, device=DEV)
+    a, b = torch.cuda.Stream(), torch.cuda.Stream()
+    ev = [torch.cuda.Event(enable_timing=True) for _ in range(3)]
+    torch.cuda.synchronize()
+    shares = []
+    for _ in range(5):
+        with torch.cuda.stream(a):
+            ev[0].record()
+            m.ops.experts(out, x, *w, ids, workspace=ws, max_ctas=98)
+            ev[1].record()
+        with torch.cuda.stream(b):
+            m.ops.permute(other, 64)
+            ev[2].record()
+        torch.cuda.synchronize()
+        shares.append(ev[0].elapsed_time(ev[2]) / ev[0].elapsed_time(ev[1]))
+    assert sorted(shares)[2] < 0.5, shares
+
+
 def test_wait_limits_do_not_count_the_predecessors_time(m):
     """The bounded waits of a GEMM give up after about a second.  That second is for its own progress: a gate/up GEMM that
     takes longer (here one CTA walks 4 million K blocks, about two seconds) must not make the down GEMM behind it give

@@ -282,6 +282,7 @@ extern "C" int b200moe_experts(void* out, const void* x, const void* w_gate, con
   g.h16 = reinterpret_cast<__nv_bfloat16*>(ws + L.hq);
   if (w8a8) g.split = MoeSplitBuffers{reinterpret_cast<float*>(ws + L.part), I32(L.cnt)};
   g.lists_ready = 1;  // the permutation's, with at least the quantisation kernel in between
+  g.hold_next = d->max_ctas > 0;  // the SMs that the cap leaves free are another stream's
   g.status = status;
   __nv_bfloat16* xg = reinterpret_cast<__nv_bfloat16*>(ws + L.xq);  // W8A16 tensor-core path: x rows in sorted order
   if (tc1_16 && do_prep) {
@@ -369,6 +370,7 @@ extern "C" int b200moe_experts(void* out, const void* x, const void* w_gate, con
     s.offsets = I32(L.s_offsets);
     s.max_mtiles = L.s_max_mtiles;
     s.max_ctas = d->max_ctas;
+    s.hold_next = g.hold_next || side;  // beside the routed experts: no SMs for CTAs that only wait
     s.P = d->T;
     s.I = (int)d->I_shared;
     s.E = 1;

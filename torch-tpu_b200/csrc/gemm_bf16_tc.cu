@@ -60,6 +60,7 @@ struct BtArgs {
   const int32_t* row_map;    // gemm2: destination row of sorted row r (NULL = r)
   int H, I, NT, m_major;
   int P;                     // rows the operand buffers hold: row ranges are clipped to it
+  int hold_next;             // no early start of the next kernel
   int bf16w;                 // weights are bf16 [E,I,H] (no scales): B tiles come straight from global memory
   __nv_bfloat16* out;        // gemm1: h [P,I]; gemm2: y rows of H
   int32_t* status;
@@ -130,7 +131,8 @@ moe_gemm_bf16_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_co
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = sh->tmem_base;
-  pdl_begin();
+  pdl_wait();
+  if (!a.hold_next) pdl_next();
 
   const int num_mtiles = *a.num_mtiles;
   const int total_tiles = num_mtiles * a.NT;
@@ -463,6 +465,7 @@ int launch_bt(const MoeGemmArgs& g, cudaStream_t st) {
   a.I = g.I;
   a.P = (int)g.P;
   a.bf16w = g.w_bf16;
+  a.hold_next = g.hold_next;
   a.NT = GEMM2 ? (g.H + 255) / 256 : g.I / 128;
   {
     const double a_bytes = (double)g.P * K * 2;

@@ -100,6 +100,7 @@ struct TcArgs {
   int32_t* part_cnt;
   int part_slot, part_rows;
   int lists_ready;  // mtiles, num_mtiles and offsets may be read before pdl_wait()
+  int hold_next;    // no early start of the next kernel
   int m_major;   // work-item order: 0 = n-tile slow, m-tile fast; 1 = m-tile slow, n-tile fast (see launch_tc)
   float* out32;  // fp32 accumulation target when KS > 1; with KS == 1 (linear layer only): fp32 rows stored instead of bf16
   // down GEMM with the weighted combine fused in: row r adds comb_w[pair] * y[r,:] into comb32[pair / div, :] (fp32,
@@ -376,7 +377,8 @@ moe_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
     }
   } else if (warp == 3) {
     // ------------------------------------------------------------------ TMA producer of the activations (one thread)
-    pdl_begin();  // (also lets the next kernel's CTAs come up as this one's leave)
+    pdl_wait();
+    if (!a.hold_next) pdl_next();  // the next kernel's CTAs come up as this one's leave
     if (lane == 0) {
       bool ok = true;
       Item nx{};
@@ -881,6 +883,7 @@ int launch_tc(const MoeGemmArgs& g, cudaStream_t st) {
   const int grid = (int)((a.part ? max_tiles * kMaxParts : max_tiles) < sms ? (a.part ? max_tiles * kMaxParts : max_tiles) : sms);
   if (grid > kMaxSplitCtas) a.part = nullptr;  // the slots are laid out for that many
   a.lists_ready = g.lists_ready;
+  a.hold_next = g.hold_next;
   return moe_launch_as(g.P <= kOverlapMaxRows, 1, moe_gemm_tc_kernel<MODE>, grid, TC_THREADS, TC_SMEM_BYTES, st, tmA, tmAs, tmB0, tmB1, a);
 }
 

@@ -57,6 +57,7 @@ struct MoeGemmArgs {
   // of that rank's buffer out_tbl[rank] (bf16 rows of H); overrides out/row_map
   const int32_t* row_src;
   const uint64_t* out_tbl;
+  int hold_next;            // tensor-core kernels: the kernel behind this one starts after it and not beside it (see pdl_next)
   int lists_ready;          // mtiles / num_mtiles / offsets are older than the launch's direct predecessor (see pdl_wait)
   int32_t* status;
 };
