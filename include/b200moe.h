@@ -50,6 +50,11 @@ enum {
                                the k additions is not fixed, so the last bit may differ from run to run.
                                Tensor-core path only (elsewhere it behaves like B200MOE_OUT_COMBINED). */
 };
+/* Which results repeat.  Batches of up to 512 (token,slot) pairs may form the down GEMM's sums with reductions whose order
+ * is not fixed.  Above that (and in b200moe_linear_w8 and b200moe_scaled_mm at every size) two calls with equal arguments
+ * give equal bits, whatever max_ctas is.  A row's last bits may still differ between batch sizes: where the tiles of a call
+ * leave most SMs idle in the last round, the last tiles of the down GEMM or the linear layer sum their K range in
+ * several parts (added in K order), and which tiles those are follows from the number of tiles. */
 
 /* stages of b200moe_experts (b200moe_experts_desc.stages) */
 enum {
@@ -189,7 +194,8 @@ typedef struct {
                          benchmark times one GEMM alone).  Any other bit is rejected. */
   int max_ctas;       /* 0 = the tensor-core GEMMs use every SM.  n > 0: their persistent grids are capped at n
                          CTAs (one per SM), which leaves the other SMs to kernels of another stream - how the
-                         expert-parallel step runs the shared expert beside its dispatch phase. */
+                         expert-parallel step runs the shared expert beside its dispatch phase.  Does not change
+                         the results. */
 } b200moe_experts_desc;
 
 size_t b200moe_experts_workspace_bytes(const b200moe_experts_desc* d);

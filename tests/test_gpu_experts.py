@@ -222,7 +222,8 @@ def test_bf16_weight_experts_multi_tile(m):
 
 def test_capped_grid_gives_the_same_result(m):
     """``max_ctas`` only changes how many persistent CTAs walk the work items: at a size without K split the
-    result is the same to the bit (and every row is written) with 1, 5 or all SMs; a negative cap is refused."""
+    result is the same to the bit (and every row is written) with 1, 5 or all SMs; a negative cap is refused.  (With
+    two K blocks no tile is shared here; shared tiles under a cap: test_gpu_tiles.py.)"""
     L = m.lib
     T, H, I, E, k = 700, 512, 256, 8, 2
     p = small_problem(T, H, I, E, k, seed=77)

@@ -76,6 +76,4 @@ def test_wait_limits_do_not_count_the_predecessors_time(m):
         assert torch.isfinite(out.float()).all(), cap
         outs.append(out)
     assert t0.elapsed_time(t1) > 2000  # (two thirds of it in the gate/up GEMM: beyond the limit, or this shows nothing)
-    # a whole tile and one cut along K sum up to 512 fp32 partial sums in other orders: a bf16 step here and there
-    a, b = outs[0].float(), outs[1].float()
-    assert float((a - b).norm()) <= 2.0 ** -9 * float(b.norm())
+    assert torch.equal(*outs)  # (which tiles are cut along K does not depend on the cap)

@@ -70,6 +70,49 @@ def test_gate_up_with_shared_tiles_is_reproducible(m):
     _close(outs[0], O.experts_w8a8(p["x"], p["ids"], p["wg"], p["wu"], p["wd"], p["sg"], p["su"], p["sd"]), "gate/up")
 
 
+def _ragged(E, T, k, seed):
+    """ids of T tokens over E experts with very uneven loads (experts without rows, one with more than one m-tile)."""
+    g = torch.Generator().manual_seed(seed)
+    p = torch.rand(E, generator=g) ** 4
+    p[0], p[1] = p.sum(), 0.0
+    return torch.stack([torch.multinomial(p, k, generator=g) for _ in range(T)]).to(torch.int32)
+
+
+@pytest.mark.parametrize("cap", [1, 7, 98, 147])
+def test_down_gemm_with_shared_tiles_and_a_capped_grid(m, cap):
+    """E <= 40 tiles of 12 K blocks on 148 SMs: the down GEMM cuts each along K.  Which tiles are cut does not depend on
+    max_ctas (a CTA then walks several parts), so every cap gives the bits of the whole grid, and a second call too."""
+    T, H, I, E, k = 300, 256, 1536, 40, 2
+    p = small_problem(T, H, I, E, k, seed=21)
+    p["ids"] = _ragged(E, T, k, 4)
+    d = to_dev(p)
+    outs = []
+    for c in (0, cap, cap):
+        out = torch.full((T, k, H), float("nan"), dtype=torch.bfloat16, device=DEV)
+        status = torch.zeros(1, dtype=torch.int32, device=DEV)
+        m.ops.experts(out, d["x"], d["wg"], d["wu"], d["wd"], d["sg"], d["su"], d["sd"], d["ids"], status=status,
+                      max_ctas=c)
+        assert int(status.item()) == 0
+        outs.append(out)
+    assert torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2])
+    _close(outs[0], O.experts_w8a8(p["x"], p["ids"], p["wg"], p["wu"], p["wd"], p["sg"], p["su"], p["sd"]), cap)
+
+
+@pytest.mark.parametrize("M,K,N", [(1, 4096, 512), (40, 2048, 1088), (130, 8192, 576)])
+def test_scaled_mm_fp32_rows_with_shared_tiles(m, M, K, N):
+    """fp32 result rows of tiles that are cut along K.  Every product of two e4m3 values is exact; tolerance as in the
+    uncut test: fp32 sums, 1e-5 of the largest result."""
+    m.load_ops()
+    g = torch.Generator().manual_seed(M)
+    x = (torch.rand(M, K, generator=g) * 2 - 1).to(torch.float8_e4m3fn)
+    y = (torch.rand(K, N, generator=g) * 2 - 1).to(torch.float8_e4m3fn)
+    outs = [torch.ops.my_ops._scaled_mm(x.to(DEV), y.t().contiguous().to(DEV), torch.tensor(0.5), torch.tensor(3.0), None,
+                                        None, torch.float32, False) for _ in range(2)]
+    assert torch.equal(*outs)
+    met = O.parity_metrics(outs[0].cpu(), x.double() @ y.double() * 1.5)
+    assert met["max_rel"] <= 1e-5 and met["cosine"] >= 0.99999, met
+
+
 @pytest.mark.parametrize("T,E,k", [(1, 4, 2), (9, 8, 2), (130, 3, 2), (700, 8, 3)])
 @pytest.mark.parametrize("I_shared", [256, 384])
 @pytest.mark.parametrize("fused", [False, True])

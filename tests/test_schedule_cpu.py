@@ -30,6 +30,13 @@ static int check(int tiles, int KB, int G, int rows) {
   }
   for (int s : seen) REQUIRE(s == 1);
   REQUIRE(longest <= (long)((tiles + G - 1) / G) * KB);
+  // fewer CTAs walk the same items: every part still has a slot of its own (its number among the parts)
+  for (int g : {1, G / 3 + 1, G}) {
+    std::vector<int> taken(G, 0);
+    for (int c = 0; c < g; ++c)
+      for (int t = c; t < p.items; t += g)
+        if (t >= p.whole) REQUIRE(t - p.whole < G && ++taken[t - p.whole] == 1);
+  }
   return 0;
 }
 int main() {

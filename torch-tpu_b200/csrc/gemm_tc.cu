@@ -95,10 +95,11 @@ struct TcArgs {
   int P;         // rows the operand buffers hold: row ranges are clipped to it
   int KS;        // K splits (down GEMM of decode-size batches); 1 = none
   // down GEMM / linear layer: tiles of a nearly empty last round are shared between CTAs (schedule.h); one slot of partial
-  // sums (part_slot floats) per CTA and one counter per shared tile, zero between launches.  NULL = tiles stay whole
+  // sums (part_slot floats) per part and one counter per shared tile, zero between launches.  NULL = tiles stay whole.
+  // The plan is made for plan_ctas CTAs whatever the cap on the grid is, so that results do not depend on max_ctas.
   float* part;
   int32_t* part_cnt;
-  int part_slot, part_rows;
+  int part_slot, part_rows, plan_ctas;
   int lists_ready;  // mtiles, num_mtiles and offsets may be read before pdl_wait()
   int hold_next;    // no early start of the next kernel
   int m_major;   // work-item order: 0 = n-tile slow, m-tile fast; 1 = m-tile slow, n-tile fast (see launch_tc)
@@ -195,7 +196,7 @@ moe_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
   const int KB_all = (GEMM2 ? a.I : a.H) / kBlock;
   // work items: (n-tile, m-tile, K split); without a K split the last ones may be parts of shared tiles
   WorkPlan plan{num_mtiles * a.NT * a.KS, 1, num_mtiles * a.NT * a.KS, KB_all};
-  if (MODE != 0 && a.part) plan = work_plan(num_mtiles * a.NT, KB_all, gridDim.x, a.part_rows);
+  if (MODE != 0 && a.part) plan = work_plan(num_mtiles * a.NT, KB_all, a.plan_ctas, a.part_rows);
   const int total_tiles = plan.items;
   const int nH = a.H / kBlock, nI = a.I / kBlock;
 
@@ -562,19 +563,19 @@ moe_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
         clear_acc();  // (a wait ran out: nothing below stores anything, but nothing reads an unset register either)
       }
       if (MODE != 0 && t >= plan.whole) {
-        // A part of a shared tile (always this CTA's last item): the partial sums go to the CTA's slot (16 bytes per lane,
-        // consecutive over the warp; only rows that exist), the CTA counts itself in, and the one that comes last adds
-        // the parts up in K order - the order of the sum does not depend on who that is - and finishes the tile.  Nobody
-        // waits for another CTA.
+        // A part of a shared tile (a CTA of the whole grid has one at most, its last item; one of a capped grid can have
+        // several): the partial sums go to the part's slot (16 bytes per lane, consecutive over the warp; only rows that
+        // exist), the CTA counts itself in, and the one that comes last adds the parts up in K order - the order of the
+        // sum does not depend on who that is - and finishes the tile.  Nobody waits for another CTA.
         if (epi_any(!ok)) {
           ok = false;
           break;
         }
-        const int first = (t - plan.whole) / plan.parts * plan.parts;  // CTA of the tile's first part
+        const int mine = t - plan.whole, first = mine / plan.parts * plan.parts;  // this part, and the tile's first one
         float4* const slots = reinterpret_cast<float4*>(a.part) + (size_t)first * (a.part_slot / 4) +
                               ((q * TC_CG + cg) * (TC_CW / 2) * 32 + lane);
         if (valid) {
-          float4* p = slots + (size_t)(blockIdx.x - first) * (a.part_slot / 4);
+          float4* p = slots + (size_t)(mine - first) * (a.part_slot / 4);
 #pragma unroll
           for (int i = 0; i < TC_CW / 2; ++i) {
             const float2 p0 = unpack2(acc[i / (TC_CW / 4)][2 * (i % (TC_CW / 4))]), p1 = unpack2(acc[i / (TC_CW / 4)][2 * (i % (TC_CW / 4)) + 1]);
@@ -597,7 +598,7 @@ moe_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
             __syncwarp();
             if (lane == 0) mbar_arrive(smem_u32(&sh->dst_empty));
           }
-          break;  // (the last item)
+          continue;
         }
         clear_acc();
         for (int c = 0; c < plan.parts; ++c) {
@@ -878,10 +879,11 @@ int launch_tc(const MoeGemmArgs& g, cudaStream_t st) {
     a.part_rows = (int)(rows < kTileM ? rows : kTileM);
   }
   const long long max_tiles = (long long)g.max_mtiles * a.NT * a.KS;
-  const int sms = g.max_ctas > 0 && g.max_ctas < device_sm_count() ? g.max_ctas : device_sm_count();
-  // (parts of shared tiles are items too)
-  const int grid = (int)((a.part ? max_tiles * kMaxParts : max_tiles) < sms ? (a.part ? max_tiles * kMaxParts : max_tiles) : sms);
-  if (grid > kMaxSplitCtas) a.part = nullptr;  // the slots are laid out for that many
+  // the whole grid (parts of shared tiles are items too), and the capped one
+  const long long items = a.part ? max_tiles * kMaxParts : max_tiles;
+  a.plan_ctas = (int)(items < device_sm_count() ? items : device_sm_count());
+  const int grid = g.max_ctas > 0 && g.max_ctas < a.plan_ctas ? g.max_ctas : a.plan_ctas;
+  if (a.plan_ctas > kMaxSplitCtas) a.part = nullptr;  // the slots are laid out for that many
   a.lists_ready = g.lists_ready;
   a.hold_next = g.hold_next;
   return moe_launch_as(g.P <= kOverlapMaxRows, 1, moe_gemm_tc_kernel<MODE>, grid, TC_THREADS, TC_SMEM_BYTES, st, tmA, tmAs, tmB0, tmB1, a);

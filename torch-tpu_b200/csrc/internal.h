@@ -4,7 +4,7 @@
 
 constexpr int kTileM = 128;  // rows of one m-tile of the grouped GEMMs
 
-// Workspace of tiles that several CTAs share (schedule.h): partial sums, one slot per CTA, and one counter per shared
+// Workspace of tiles that several CTAs share (schedule.h): partial sums, one slot per part, and one counter per shared
 // tile, zero when the launch starts and zero again when it ends.
 constexpr int kMaxSplitCtas = 160;
 constexpr int kSplitCounters = kMaxSplitCtas;

@@ -4,7 +4,8 @@
 // `tiles` output tiles of KB K blocks each are dealt out to G CTAs in rounds, item t to CTA t % G.  When tiles is just
 // above a multiple of G the last round leaves most CTAs idle (192 tiles on 148 SMs: 44 of them work on the second round).
 // Then each of the last `rem` tiles is cut along K into `parts` items, one per CTA, and the CTA that finishes a tile's last
-// part adds the partial sums up.
+// part adds the partial sums up.  A cut tile sums its K range in other groups than a whole one, so an output row's last
+// bits depend on whether its tile is cut: on the number of tiles (the batch), but not on how many CTAs walk the items.
 #pragma once
 #include <stdint.h>
 
