@@ -40,7 +40,9 @@ static inline bool moe_aligned16(const void* p) { return (reinterpret_cast<uintp
 // before it touches memory that an earlier kernel of the stream writes or reads (it returns when the predecessor has
 // completed and its writes are visible), and pdl_next(), which lets the successor start, comes after it.  So when a
 // kernel starts, everything before its direct predecessor is complete.  Launched after anything else than such a
-// kernel, pdl_wait() finds its predecessor complete.
+// kernel, pdl_wait() finds its predecessor complete.  Such a kernel reads through plain pointers: `const __restrict__`
+// would promise that the data does not change while the kernel runs (and allow the read-only load path), and it runs
+// while its predecessor still writes.
 // A kernel whose SMs are meant to be shared with another stream's leaves pdl_next() out (the GEMMs' hold_next): started
 // early, the blocks behind it take SMs and wait there.  With 98 CTAs the gate/up GEMM of one Mixtral expert, 4096 tokens,
 // held a permutation of another stream until its own end: it ended 758 us after the call's start, 88 us without (the call

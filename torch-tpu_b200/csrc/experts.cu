@@ -103,8 +103,8 @@ WsLayout make_layout(const b200moe_experts_desc& d) {
   return L;
 }
 
-__global__ void scales_to_f32_kernel(float* __restrict__ dst, const __nv_bfloat16* __restrict__ a,
-                                     const __nv_bfloat16* __restrict__ b, const __nv_bfloat16* __restrict__ c, int64_t n) {
+__global__ void scales_to_f32_kernel(float* __restrict__ dst, const __nv_bfloat16* a,
+                                     const __nv_bfloat16* b, const __nv_bfloat16* c, int64_t n) {
   pdl_begin();
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) {
@@ -600,7 +600,7 @@ LinLayout lin_layout(int64_t M, int64_t K, int64_t N, int scale_dtype) {
   L.total = o;
   return L;
 }
-__global__ void scales1_to_f32_kernel(float* __restrict__ dst, const __nv_bfloat16* __restrict__ s, int64_t n) {
+__global__ void scales1_to_f32_kernel(float* __restrict__ dst, const __nv_bfloat16* s, int64_t n) {
   pdl_begin();
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) dst[i] = __bfloat162float(s[i]);
@@ -666,7 +666,7 @@ extern "C" int b200moe_linear_w8(void* out, const void* x, const void* w, const 
 
 // ---- FP8 x FP8 matrix product with one scale per operand ------------------------------------------------------------
 namespace {
-__global__ void fill_scalar_scale_kernel(float* __restrict__ dst, const float* __restrict__ scale, int64_t n) {
+__global__ void fill_scalar_scale_kernel(float* __restrict__ dst, const float* scale, int64_t n) {
   pdl_begin();
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) dst[i] = scale ? *scale : 1.0f;

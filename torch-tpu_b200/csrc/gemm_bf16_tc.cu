@@ -490,8 +490,8 @@ int launch_bt(const MoeGemmArgs& g, cudaStream_t st) {
 
 // gather of bf16 rows into sorted order: dst[r,:] = x[row_map[r] / div, :] (16-byte accesses; one warp per row)
 __global__ void __launch_bounds__(256)
-gather_rows_bf16_kernel(__nv_bfloat16* __restrict__ dst, const __nv_bfloat16* __restrict__ x,
-                        const int32_t* __restrict__ row_map, int div, int64_t rows, int H) {
+gather_rows_bf16_kernel(__nv_bfloat16* __restrict__ dst, const __nv_bfloat16* x,
+                        const int32_t* row_map, int div, int64_t rows, int H) {
   pdl_begin();
   const int lane = threadIdx.x & 31;
   const int64_t r = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
@@ -500,7 +500,18 @@ gather_rows_bf16_kernel(__nv_bfloat16* __restrict__ dst, const __nv_bfloat16* __
   if (pr < 0) return;  // position of a dropped pair
   const uint4* src = reinterpret_cast<const uint4*>(x + (int64_t)(pr / div) * H);
   uint4* d = reinterpret_cast<uint4*>(dst + r * H);
-  for (int c = lane; c < H / 8; c += 32) d[c] = src[c];
+  // eight loads are issued before the first store (a store could be to the row that the next load reads, for all the
+  // compiler knows, so it does not move loads up by itself)
+  constexpr int U = 8;
+  for (int c0 = lane; c0 < H / 8; c0 += U * 32) {
+    uint4 v[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (c0 + u * 32 < H / 8) v[u] = src[c0 + u * 32];
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (c0 + u * 32 < H / 8) d[c0 + u * 32] = v[u];
+  }
 }
 
 }  // namespace

@@ -202,7 +202,7 @@ __global__ void __launch_bounds__(256) gemm2_simple_kernel(MoeGemmArgs a) {
 
 __global__ void __launch_bounds__(1024)
 build_mtiles_kernel(int32_t* __restrict__ mtiles, int32_t* __restrict__ num_mtiles,
-                    const int32_t* __restrict__ offsets, int E, int max_rows, int max_mtiles, int32_t* split_cnt) {
+                    const int32_t* offsets, int E, int max_rows, int max_mtiles, int32_t* split_cnt) {
   pdl_begin();
   moe_clear_counters(split_cnt);
   __shared__ int tmp[1024];
@@ -240,9 +240,9 @@ __global__ void __launch_bounds__(256) identity_lists_kernel(MoeIdentityLists li
 // one memory round trip per slot (Qwen3 shape, 8192 tokens x 8 slots, 300 MB: 68 -> 54 us).
 constexpr int CB_SLOTS = 4;
 __global__ void __launch_bounds__(256)
-combine_kernel(__nv_bfloat16* __restrict__ out, const __nv_bfloat16* __restrict__ y, const void* __restrict__ w,
-               int w_dtype, const __nv_bfloat16* __restrict__ add, const int32_t* __restrict__ pos,
-               const int32_t* __restrict__ ids, int E, int64_t T, int k, int H) {
+combine_kernel(__nv_bfloat16* __restrict__ out, const __nv_bfloat16* y, const void* w,
+               int w_dtype, const __nv_bfloat16* add, const int32_t* pos,
+               const int32_t* ids, int E, int64_t T, int k, int H) {
   pdl_begin();
   const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int hv = H / 8;

@@ -897,7 +897,7 @@ bool moe_tc_available() {
 }
 
 namespace {
-__global__ void f32_rows_to_bf16_kernel(__nv_bfloat16* __restrict__ out, const float* __restrict__ in, int64_t n) {
+__global__ void f32_rows_to_bf16_kernel(__nv_bfloat16* __restrict__ out, const float* in, int64_t n) {
   pdl_begin();
   const int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * 4;
   if (i + 3 < n) {

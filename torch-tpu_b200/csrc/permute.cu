@@ -18,7 +18,7 @@ constexpr int kMaxDevices = 64;  // per-device caches below are indexed by the C
 
 // Per-warp histogram of this chunk in shared memory: wh[w*E + e].  Returns the pair's expert (or -1)
 // and its rank among equal experts in lower lanes of its warp.
-__device__ __forceinline__ int chunk_hist(const int32_t* __restrict__ ids, int64_t P, int E, int64_t p,
+__device__ __forceinline__ int chunk_hist(const int32_t* ids, int64_t P, int E, int64_t p,
                                           int* wh, int& rank_in_warp, int32_t* status) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   for (int i = threadIdx.x; i < 32 * E; i += blockDim.x) wh[i] = 0;
@@ -39,7 +39,7 @@ __device__ __forceinline__ int chunk_hist(const int32_t* __restrict__ ids, int64
 }
 
 __global__ void __launch_bounds__(kChunk)
-permute_hist_kernel(const int32_t* __restrict__ ids, int64_t P, int E, int32_t* __restrict__ chunk_cnt,
+permute_hist_kernel(const int32_t* ids, int64_t P, int E, int32_t* __restrict__ chunk_cnt,
                     int32_t* status) {
   pdl_begin();
   extern __shared__ int wh[];
@@ -116,8 +116,8 @@ permute_scan_kernel(int32_t* __restrict__ chunk_cnt, int nchunks, int E, int32_t
 }
 
 __global__ void __launch_bounds__(kChunk)
-permute_scatter_kernel(const int32_t* __restrict__ ids, int64_t P, int E,
-                       const int32_t* __restrict__ chunk_base, const int32_t* __restrict__ offsets,
+permute_scatter_kernel(const int32_t* ids, int64_t P, int E,
+                       const int32_t* chunk_base, const int32_t* offsets,
                        int32_t* __restrict__ sorted_pair, int32_t* __restrict__ pos_of) {
   pdl_begin();
   extern __shared__ int wh[];
@@ -147,7 +147,7 @@ permute_scatter_kernel(const int32_t* __restrict__ ids, int64_t P, int E,
 
 // P <= 1024: histogram, scan and scatter in one CTA
 __global__ void __launch_bounds__(kChunk)
-permute_small_kernel(const int32_t* __restrict__ ids, int64_t P, int E, int32_t* __restrict__ offsets,
+permute_small_kernel(const int32_t* ids, int64_t P, int E, int32_t* __restrict__ offsets,
                      int32_t* __restrict__ sorted_pair, int32_t* status, int32_t* __restrict__ mtiles,
                      int32_t* __restrict__ num_mtiles, int max_mtiles, int32_t* __restrict__ pos_of,
                      int32_t* split_cnt) {
@@ -183,7 +183,7 @@ permute_small_kernel(const int32_t* __restrict__ ids, int64_t P, int E, int32_t*
 // list)
 constexpr int kMaxCluster = 8;  // portable cluster size
 __global__ void __launch_bounds__(kChunk)
-permute_cluster_kernel(const int32_t* __restrict__ ids, int64_t P, int E, int32_t* __restrict__ offsets,
+permute_cluster_kernel(const int32_t* ids, int64_t P, int E, int32_t* __restrict__ offsets,
                        int32_t* __restrict__ sorted_pair, int32_t* status, int32_t* __restrict__ mtiles,
                        int32_t* __restrict__ num_mtiles, int max_mtiles, int32_t* __restrict__ pos_of, int32_t* split_cnt) {
   pdl_begin();
@@ -240,8 +240,8 @@ permute_cluster_kernel(const int32_t* __restrict__ ids, int64_t P, int E, int32_
 __global__ void gather_scatter_index_kernel(int32_t* __restrict__ gather_index,
                                             int32_t* __restrict__ scatter_index,
                                             int32_t* __restrict__ num_per_expert,
-                                            const int32_t* __restrict__ sorted_pair,
-                                            const int32_t* __restrict__ offsets, int64_t T, int k) {
+                                            const int32_t* sorted_pair,
+                                            const int32_t* offsets, int64_t T, int k) {
   pdl_begin();
   const int e = blockIdx.x;
   const int b = offsets[e], n = offsets[e + 1] - b;
@@ -260,7 +260,7 @@ __global__ void gather_scatter_index_kernel(int32_t* __restrict__ gather_index,
 // warp walks a whole row (fewer blocks, the row's gather index read once).
 __global__ void __launch_bounds__(256)
 quant_rows_kernel(uint8_t* __restrict__ q, float* __restrict__ s_t, int64_t ld,
-                  const __nv_bfloat16* __restrict__ x, const int32_t* __restrict__ row_map, int div,
+                  const __nv_bfloat16* x, const int32_t* row_map, int div,
                   int64_t rows, int H, int cpw, int warps_per_row, MoeIdentityLists lists) {
   pdl_begin();
   if (lists.offsets && blockIdx.x == 0) moe_write_identity_lists(lists, (int)rows);
@@ -320,8 +320,8 @@ quant_rows_kernel(uint8_t* __restrict__ q, float* __restrict__ s_t, int64_t ld,
 // row; a warp takes `cpw` 512-column chunks of a token, their loads issued together.
 constexpr int QT_CPW = 2;
 __global__ void __launch_bounds__(256)
-quant_tokens_kernel(uint8_t* __restrict__ q, float* __restrict__ s_t, int64_t ld, const __nv_bfloat16* __restrict__ x,
-                    const int32_t* __restrict__ pos_of, int64_t T, int k, int H, int cpw, int warps_per_tok,
+quant_tokens_kernel(uint8_t* __restrict__ q, float* __restrict__ s_t, int64_t ld, const __nv_bfloat16* x,
+                    const int32_t* pos_of, int64_t T, int k, int H, int cpw, int warps_per_tok,
                     float* __restrict__ acc32) {
   pdl_begin();
   const int lane = threadIdx.x & 31;

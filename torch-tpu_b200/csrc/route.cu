@@ -121,7 +121,7 @@ __device__ __forceinline__ void group_mask(float (&v)[VPT], int n, int n_groups,
 
 template <int VPT>
 __global__ void __launch_bounds__(kWarpsPerBlock * 32)
-topk_kernel(void* __restrict__ values, int32_t* __restrict__ indices, const void* __restrict__ scores,
+topk_kernel(void* __restrict__ values, int32_t* __restrict__ indices, const void* scores,
             int dtype, int64_t batch, int n, int n_groups, int topk_groups, int k) {
   pdl_begin();
   const int lane = threadIdx.x & 31;
@@ -218,7 +218,7 @@ __device__ __forceinline__ void route_row(float (&s)[VPT], const RouteArgs& a, i
 
 template <int VPT>
 __global__ void __launch_bounds__(kWarpsPerBlock * 32)
-route_kernel(const float* __restrict__ logits, int64_t T, int n, const RouteArgs a) {
+route_kernel(const float* logits, int64_t T, int n, const RouteArgs a) {
   pdl_begin();
   const int lane = threadIdx.x & 31;
   const int64_t row = (int64_t)blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
@@ -280,8 +280,8 @@ __device__ __forceinline__ void cp_async16(void* smem_dst, const void* gsrc, int
 // grid (ceil(T / BM), ceil(E / BN))
 template <class C>
 __global__ void __launch_bounds__(C::THREADS)
-router_gemm_kernel(float* __restrict__ logits, const __nv_bfloat16* __restrict__ x,
-                   const __nv_bfloat16* __restrict__ wr, int64_t T, int64_t H, int64_t E) {
+router_gemm_kernel(float* __restrict__ logits, const __nv_bfloat16* x,
+                   const __nv_bfloat16* wr, int64_t T, int64_t H, int64_t E) {
   pdl_begin();
   extern __shared__ __align__(16) uint8_t rg_smem[];
   __nv_bfloat16* const stages = reinterpret_cast<__nv_bfloat16*>(rg_smem);
@@ -364,8 +364,8 @@ router_gemm_kernel(float* __restrict__ logits, const __nv_bfloat16* __restrict__
 // experts, so the read of the router weights is spread over many SMs and only H/1024 loads deep.
 constexpr int RV_MAXT = 8;
 __global__ void __launch_bounds__(128)
-router_gemv_kernel(float* __restrict__ logits, const __nv_bfloat16* __restrict__ x,
-                   const __nv_bfloat16* __restrict__ wr, int64_t T, int64_t H, int64_t E) {
+router_gemv_kernel(float* __restrict__ logits, const __nv_bfloat16* x,
+                   const __nv_bfloat16* wr, int64_t T, int64_t H, int64_t E) {
   pdl_begin();
   __shared__ float part[4][RV_MAXT];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -412,8 +412,8 @@ constexpr int RS_TOK = 4, RS_WARPS = 8;
 // has just formed: one launch less in front of the experts (Mixtral shape, 32 tokens: 6.6 + 3.5 us as two kernels).
 template <int EP, bool ROUTE>
 __global__ void __launch_bounds__(RS_WARPS * 32)
-router_small_e_kernel(float* __restrict__ logits, const __nv_bfloat16* __restrict__ x,
-                       const __nv_bfloat16* __restrict__ wr, int64_t T, int64_t H, int E, const RouteArgs ra) {
+router_small_e_kernel(float* __restrict__ logits, const __nv_bfloat16* x,
+                       const __nv_bfloat16* wr, int64_t T, int64_t H, int E, const RouteArgs ra) {
   pdl_begin();
   __shared__ float sums[RS_TOK][EP];
   __shared__ float part[RS_WARPS][RS_TOK][EP];
