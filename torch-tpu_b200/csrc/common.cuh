@@ -48,12 +48,16 @@ static inline bool moe_aligned16(const void* p) { return (reinterpret_cast<uintp
 // held a permutation of another stream until its own end: it ended 758 us after the call's start, 88 us without (the call
 // itself 1.16 and 1.14 ms).  DeepSeek shape, 1 token, the shared expert's GEMMs on the side stream: 136 -> 115 us; 8 to 64
 // tokens the same with either.
-// Not for large problems: there the gaps are nothing and the early starts cost more than they give (every launch
-// overlapped / only those below the line: Mixtral shape, 4096 tokens 2074 / 2045 us, Qwen3 shape, 8192 tokens 636 / 631;
-// Qwen3 experts op, 777 tokens, all below it: 166 us, 178 with none).  The line is drawn at the number of blocks, and for
-// the persistent GEMMs at the number of rows.
-constexpr long long kOverlapMaxBlocks = 1024;
-constexpr int64_t kOverlapMaxRows = 8191;
+// Not for large launches: what an early start saves is a gap of two or three microseconds, whatever the size, and beside
+// a long kernel it costs more than that.  Layer times in us, without / with the early start:
+//   GEMMs, by the K blocks (0.5 to 0.6 us each) that a CTA of the gate/up GEMM walks: 15 (small layer, 4096 tokens) 69.9 /
+//   63.9; 73 (Qwen3 shape, 1024) 113.4 / 110.5; 124 (2048) 192.9 / 186.2; 207 (4096) 332 / 331; 290 (Mixtral shape, 512)
+//   428 / 430; 484 (1024) 635 / 641; 872 (2048) 1103 / 1124; 1646 (4095) 1976 / 2024.
+//   Other kernels, by their blocks: up to 512 (small layer, 512 tokens) 36.9 / 34.8; 2048 (combine, small layer, 4096
+//   tokens) 63.9 / 62.8 and (Qwen3 shape, 2048) 186.2 / 183.5; 4096 (Qwen3 shape, 4096) 331 / 335.
+constexpr long long kOverlapMaxBlocks = 2048;
+constexpr int64_t kOverlapMaxKBlocks = 256;  // per CTA of a GEMM
+constexpr int64_t kOverlapMaxRowsPerExpert = 16;
 #ifdef __CUDACC__
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }

@@ -485,7 +485,7 @@ int launch_bt(const MoeGemmArgs& g, cudaStream_t st) {
   const long long max_tiles = (long long)g.max_mtiles * a.NT;
   const int sms = g.max_ctas > 0 && g.max_ctas < moe_device_sm_count() ? g.max_ctas : moe_device_sm_count();
   const int grid = (int)(max_tiles < sms ? max_tiles : sms);
-  return moe_launch_as(g.P <= kOverlapMaxRows, 1, moe_gemm_bf16_tc_kernel<GEMM2>, grid, BT_THREADS, BT_SMEM_BYTES, st, tmA, tmB0, tmB1, a);
+  return moe_launch_as(moe_gemm_overlaps(g, a.NT, K, grid), 1, moe_gemm_bf16_tc_kernel<GEMM2>, grid, BT_THREADS, BT_SMEM_BYTES, st, tmA, tmB0, tmB1, a);
 }
 
 // gather of bf16 rows into sorted order: dst[r,:] = x[row_map[r] / div, :] (16-byte accesses; one warp per row)

@@ -886,7 +886,7 @@ int launch_tc(const MoeGemmArgs& g, cudaStream_t st) {
   if (a.plan_ctas > kMaxSplitCtas) a.part = nullptr;  // the slots are laid out for that many
   a.lists_ready = g.lists_ready;
   a.hold_next = g.hold_next;
-  return moe_launch_as(g.P <= kOverlapMaxRows, 1, moe_gemm_tc_kernel<MODE>, grid, TC_THREADS, TC_SMEM_BYTES, st, tmA, tmAs, tmB0, tmB1, a);
+  return moe_launch_as(moe_gemm_overlaps(g, a.NT, K, grid), 1, moe_gemm_tc_kernel<MODE>, grid, TC_THREADS, TC_SMEM_BYTES, st, tmA, tmAs, tmB0, tmB1, a);
 }
 
 }  // namespace
