@@ -71,6 +71,16 @@ def test_workspace_bytes(m):
         ops.make_desc(16, 7168, 2048, 256, 8, out_mode=m.lib.OUT_COMBINED))
 
 
+def test_workspace_partial_sums_share_one_region(m):
+    """The fused combine's rows, the rows of a K-split down GEMM and the slots of shared tiles (160 of 128 x 256 fp32) are
+    never in use together: the largest of them is what a workspace has room for."""
+    ops, T, H, k = m.ops, 4096, 4096, 2
+    n = {mode: ops.experts_workspace_bytes(ops.make_desc(T, H, 14336, 8, k, out_mode=mode))
+         for mode in (m.lib.OUT_PER_SLOT, m.lib.OUT_COMBINED, m.lib.OUT_COMBINED_FUSED)}
+    assert n[m.lib.OUT_COMBINED] - n[m.lib.OUT_PER_SLOT] == T * k * H * 2              # the per-slot rows, nothing else
+    assert n[m.lib.OUT_COMBINED_FUSED] - n[m.lib.OUT_COMBINED] == T * H * 4 - 160 * 128 * 256 * 4
+
+
 def test_workspace_bytes_never_shrink_with_tokens(m):
     """A layer sizes its workspace once for max_tokens and then runs any smaller batch in it."""
     ops = m.ops

@@ -2,6 +2,8 @@
 // -> grouped down GEMM -> scatter or weighted combine, all enqueued on one stream into a caller-owned
 // workspace.  Stands in for tpudnnFusedMoEFusedExpertsMultiCoreAsync
 // (third_party/tpuDNN/include/tpuDNNTensor.h:1585-1611) and the PPL kernel my_ops/fusedMoE.pl:795-810.
+#include <algorithm>
+
 #include "internal.h"
 
 namespace {
@@ -75,12 +77,13 @@ WsLayout make_layout(const b200moe_experts_desc& d) {
   const int64_t acc_tokens = d.out_mode == B200MOE_OUT_COMBINED_FUSED ? d.T
                              : d.out_mode == B200MOE_OUT_COMBINED     ? (d.T < kSplitMaxPairs ? d.T : kSplitMaxPairs)
                                                                       : 0;
-  L.acc32 = take(w8a8 ? (size_t)acc_tokens * d.H * sizeof(float) : 0);
-  // fp32 partial sums of the K-split down GEMM (decode-size batches only)
-  // (sized for min(P, limit) rows whatever P is, so that the workspace size never shrinks when T grows)
-  L.y32 = take(w8a8 ? (size_t)(P < kSplitMaxPairs ? P : kSplitMaxPairs) * d.H * sizeof(float) : 0);
-  // partial sums and counters of tiles that CTAs share
-  L.part = take(w8a8 ? moe_split_part_bytes(P) : 0);
+  // One region for three things of which a call has one at most: the fused combine's rows; the fp32 partial sums of a down
+  // GEMM whose K is split without it (decode-size batches only; sized for min(P, limit) rows whatever P is, so that the
+  // workspace size never shrinks when T grows); and the partial sums of tiles that CTAs share, where K is not split and
+  // the combine not fused.
+  const size_t y32_bytes = (size_t)(P < kSplitMaxPairs ? P : kSplitMaxPairs) * d.H * sizeof(float);
+  L.acc32 = L.y32 = L.part =
+      take(w8a8 ? std::max({(size_t)acc_tokens * d.H * sizeof(float), y32_bytes, moe_split_part_bytes(P)}) : 0);
   L.cnt = take(kSplitCounters * sizeof(int32_t));
   // fp32 copies of bf16 block scales (the tensor-core kernels read fp32 scales only)
   L.sc32 = take(d.scale_dtype == B200MOE_BF16 && w8a8 ? 3 * (size_t)d.E * nI * nH * sizeof(float) : 0);
@@ -94,8 +97,8 @@ WsLayout make_layout(const b200moe_experts_desc& d) {
     L.s_hq = take(w8a8 ? (size_t)d.T * d.I_shared : (size_t)d.T * d.I_shared * 2);
     L.s_hs = take(w8a8 ? nIs * (size_t)L.lds * sizeof(float) : 0);
     L.s_y = take((size_t)d.T * d.H * 2);
-    L.s_y32 = take(w8a8 ? (size_t)(d.T < kSplitMaxPairs ? d.T : kSplitMaxPairs) * d.H * sizeof(float) : 0);
-    L.s_part = take(w8a8 ? moe_split_part_bytes(d.T) : 0);
+    const size_t s_y32_bytes = (size_t)(d.T < kSplitMaxPairs ? d.T : kSplitMaxPairs) * d.H * sizeof(float);
+    L.s_y32 = L.s_part = take(w8a8 ? std::max(s_y32_bytes, moe_split_part_bytes(d.T)) : 0);
     L.s_cnt = take(kSplitCounters * sizeof(int32_t));
     L.s_sc32 = take(d.scale_dtype == B200MOE_BF16 && w8a8 ? 3 * nIs * nH * sizeof(float) : 0);
   }
