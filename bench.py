@@ -233,8 +233,10 @@ def median(v):
 
 
 def launches_per_step(wl, T, world=1, ep="nccl"):
+    import torch
     P = T * wl["k"]
-    route = 1 if wl["E"] <= 16 and 16 < T <= 592 else 2  # router and selection (one kernel for few experts and tokens)
+    # router and selection: one kernel for few experts while its blocks of four tokens fit the SMs at once
+    route = 1 if wl["E"] <= 16 and 16 < T <= 4 * torch.cuda.get_device_properties(0).multi_processor_count else 2
     sort = lambda pairs: 1 if pairs <= 8192 else 3
     if world > 1 and ep == "p2p":
         # router, route, permute | counts exchange, plan, dispatch, barrier | scales, tiles, 2 GEMMs, barrier | combine

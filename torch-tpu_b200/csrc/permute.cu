@@ -478,7 +478,7 @@ int moe_quant_tokens(uint8_t* q, float* s_t, int64_t ld, const void* x, const in
                      int64_t H, float* acc32, cudaStream_t st) {
   const int64_t chunks = (H + 511) / 512;
   // two chunks per warp once that still leaves every SM its full set of warps
-  const int cpw = T * chunks >= 2 * 64 * 148 ? QT_CPW : 1;
+  const int cpw = T * chunks >= (int64_t)QT_CPW * 64 * moe_device_sm_count() ? QT_CPW : 1;
   const int64_t wpt = (chunks + cpw - 1) / cpw;
   return moe_launch(quant_tokens_kernel, (unsigned)((T * wpt + 7) / 8), 256, 0, st, q, s_t, ld,
                     reinterpret_cast<const __nv_bfloat16*>(x), pos_of, T, (int)k, (int)H, cpw, (int)wpt, acc32);
