@@ -1,6 +1,6 @@
 """Edges of the tensor-core GEMMs' work split: rows per tile around the small activation boxes (16, 32) and the full tile,
-tiles that several CTAs share along K, the shared expert walked as one more expert of the same launches, and the
-kernels in front of them (fused router + selection, the cluster permutation)."""
+tiles that several CTAs share along K (linear layer, scaled product, down GEMM), the shared expert's pass, and the kernels
+in front of them (fused router + selection, the cluster permutation)."""
 import pytest
 import torch
 
@@ -57,7 +57,9 @@ def test_linear_with_shared_tiles(m, M, K, N):
     assert float(err) <= 4 * 2.0 ** -8 + 5e-3, float(err)
 
 
-def test_gate_up_with_shared_tiles_is_reproducible(m):
+def test_few_tokens_with_a_long_gate_up_k_loop_are_reproducible(m):
+    """Six tokens, 32 K blocks in the gate/up GEMM and two in the down GEMM (neither cuts a tile or splits K): calls give
+    equal bits.  Cut tiles: test_down_gemm_with_shared_tiles_and_a_capped_grid, test_linear_with_shared_tiles."""
     H, I, E, T = 4096, 256, 4, 6
     p = small_problem(T, H, I, E, 2, seed=8)
     d = to_dev(p)
@@ -116,9 +118,9 @@ def test_scaled_mm_fp32_rows_with_shared_tiles(m, M, K, N):
 @pytest.mark.parametrize("T,E,k", [(1, 4, 2), (9, 8, 2), (130, 3, 2), (700, 8, 3)])
 @pytest.mark.parametrize("I_shared", [256, 384])
 @pytest.mark.parametrize("fused", [False, True])
-def test_shared_expert_merged_and_beside(m, T, E, k, I_shared, fused):
-    """I_shared = I: one more expert of the launches; another size: a pass of its own.  Also with an id out of range,
-    whose dropped row must not move the shared expert's."""
+def test_shared_expert_beside_and_in_line(m, T, E, k, I_shared, fused):
+    """The shared expert, of the routed experts' size and of another: beside them on a side stream (up to 64 tokens) or
+    behind them.  Also with an id out of range, whose dropped row must not move the shared expert's."""
     H, I = 512, 256
     p = small_problem(T, H, I, E, k, seed=T + E)
     sh = O.make_expert_weights(1, H, I_shared, seed=99)
@@ -151,6 +153,23 @@ def test_router_route_is_the_two_calls(m, T, E, k):
         assert torch.equal(ids, want[0]) and torch.equal(w, want[1])
         ref = x.double() @ wr.double().T
         assert float((logits.double() - ref).abs().max()) <= 2e-6 * float(ref.abs().max())
+
+
+@pytest.mark.parametrize("T", [17, 64, 591, 592, 593, 600])
+@pytest.mark.parametrize("E,k,groups,topk_groups", [(8, 2, 1, 1), (16, 4, 4, 2), (64, 6, 8, 3)])
+def test_router_route_with_groups_and_around_one_block_per_sm(m, T, E, k, groups, topk_groups):
+    """Up to 4 tokens per SM (592) and 16 experts one kernel routes too, above that a second one: the same logits, ids and
+    weights as the two calls, with groups as well."""
+    H = 256
+    x, wr, _ = O.make_inputs(T, H, E, seed=T + E, router_std=H ** -0.5)
+    x, wr = x.to(DEV), wr.to(DEV)
+    bias = torch.randn(E, generator=torch.Generator().manual_seed(2)).to(DEV) * 0.1
+    for score, b in (("softmax", None), ("sigmoid", bias)):
+        logits = torch.full((T, E), float("nan"), device=DEV)
+        ids, w = m.ops.router_route(x, wr, k, score, b, groups, topk_groups, True, 1.5, logits=logits)
+        assert torch.equal(logits, m.ops.router_logits(x, wr))
+        want = m.ops.route(logits, k, score, b, groups, topk_groups, True, 1.5)
+        assert torch.equal(ids, want[0]) and torch.equal(w, want[1])
 
 
 @pytest.mark.parametrize("P,E", [(1024, 8), (1025, 8), (2048, 1000), (8191, 128), (8192, 1024), (8193, 64)])
