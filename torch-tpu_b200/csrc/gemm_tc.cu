@@ -179,7 +179,8 @@ moe_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
   // The A stages start as zeros.  A tile of at most 32 rows loads only the one or two 16-row boxes it needs, so the other
   // rows of its MMAs multiply zeros (or an earlier tile's rows) instead of the next experts' rows: this part runs at its
   // power limit even where it only streams weights, and the tensor cores' switching on rows nobody asked for came out of
-  // the clock (DeepSeek shape, 64 tokens: 1410 -> 1530 MHz, layer 1.78 -> 1.64 ms; Mixtral shape, 1 token: 106 -> 95 us).
+  // the clock (layers, 128-row box for every tile / as it is, timed in turn: DeepSeek shape, 64 tokens 1815 / 1709 us, SM
+  // clock 1425 / 1590 MHz; Mixtral shape, 1 token 102.0 / 95.2 us, 32 tokens 277 / 272).
   // Taller tiles take the one 128-row box: four or more small boxes per K block cost more than they saved (DeepSeek
   // shape, 2048 tokens, 64 rows per expert: 2.60 -> 2.70 ms).
   for (int i = threadIdx.x; i < TC_STAGES * (TC_A_BYTES / 16); i += TC_THREADS)
@@ -637,7 +638,7 @@ moe_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
       // several thousand cycles per tile.  Each warp turns its own 32 rows x TC_CW columns through a private patch of
       // shared memory instead (16-byte chunks, XOR-swizzled so that neither side has bank conflicts; only warp-level
       // synchronisation) and then stores whole 64- or 128-byte row segments per group of lanes.  (Handing each row's
-      // 128 bytes to the copy engine, so that the warp could go on, was slower: Qwen3 down GEMM 217 -> 241 us.)
+      // 128 bytes to the copy engine, so that the warp could go on, was slower: Qwen3 down GEMM 196 -> 241 us.)
       static_assert(TC_CW == 64, "the row-segment stores below are laid out for 64 columns per warp");
       const int wepi = warp - 4;
       if (MODE == 0) {

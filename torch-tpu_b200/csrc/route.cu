@@ -1,6 +1,6 @@
 // Routing kernels: plain / grouped top-k on given scores, the fused score->select->normalise chain,
 // and the router GEMM.  One warp owns one row; element e of the row lives in lane e%32, register e/32,
-// so loads are coalesced and every selection step is a register scan plus five shuffles.
+// so loads are coalesced and every selection step is a register scan plus two warp reductions.
 //
 // Tie rule everywhere: among equal values the LOWEST index wins (the reference leaves tie order open:
 // aten::topk on its CPU path and an index-perturbation on its device path, native_ops/Topk.pl:82-100).
