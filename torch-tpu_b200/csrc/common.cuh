@@ -51,9 +51,9 @@ static inline bool moe_aligned16(const void* p) { return (reinterpret_cast<uintp
 // Not for large launches: what an early start saves is a gap of two or three microseconds, whatever the size, and beside
 // a long kernel it costs more than that.  Layer times in us, without / with the early start:
 //   GEMMs, by the K blocks (0.5 to 0.6 us each) that a CTA of the gate/up GEMM walks: 15 (small layer, 4096 tokens) 69.9 /
-//   63.9; 73 (Qwen3 shape, 1024) 113.4 / 110.5; 124 (2048) 192.9 / 186.2; 207 (4096) 332 / 331; 290 (Mixtral shape, 512)
-//   428 / 430; 484 (1024) 635 / 641; 872 (2048) 1103 / 1124; 1646 (4095) 1976 / 2024.
-//   Other kernels, by their blocks: up to 512 (small layer, 512 tokens) 36.9 / 34.8; 2048 (combine, small layer, 4096
+//   63.9; 83 (Qwen3 shape, 1024) 113.4 / 110.5; 125 (2048) 192.9 / 186.2; 208 (4096) 332 / 331; 303 (Mixtral shape, 512)
+//   428 / 430; 496 (1024) 635 / 641; 884 (2048) 1103 / 1124; 1647 (4095) 1976 / 2024.
+//   Other kernels, by their blocks: up to 256 (small layer, 512 tokens) 36.9 / 34.8; 2048 (combine, small layer, 4096
 //   tokens) 63.9 / 62.8 and (Qwen3 shape, 2048) 186.2 / 183.5; 4096 (Qwen3 shape, 4096) 331 / 335.
 constexpr long long kOverlapMaxBlocks = 2048;
 constexpr int64_t kOverlapMaxKBlocks = 256;  // per CTA of a GEMM
